@@ -1123,6 +1123,8 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
     }
     P.tf_lo = tf->lo;
     P.tf_hi = tf->hi;
+    P.tf_rcp = vrc::tf_reciprocal(tf->lo, tf->hi);
+    P.tf_wm1 = float(P.tf_width - 1);
     const size_t npix = (size_t)p->width * p->height;
     cudaStream_t s = ctx->stream;
     VRC_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));

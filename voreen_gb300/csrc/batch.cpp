@@ -153,6 +153,8 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
         R.P.tf_width = it.tf->width;
         R.P.tf_lo = it.tf->lo;
         R.P.tf_hi = it.tf->hi;
+        R.P.tf_rcp = vrc::tf_reciprocal(it.tf->lo, it.tf->hi);
+        R.P.tf_wm1 = float(R.P.tf_width - 1);
         R.P.out = it.out;
         R.P.out_format = it.out_format;
         if (it.params.empty_space_skipping) {

@@ -100,21 +100,29 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS)
         const int py = P.ry0 + ty * (32 >> P.tile_wshift) + (lane >> P.tile_wshift);
         if (px < P.rx1 && py < P.ry1) {
             float4 f, l;
-            analytic_entry_exit(P, px, py, f, l);
-            const bool bg = f.x == 0.f && f.y == 0.f && f.z == 0.f && f.w == 0.f && l.x == 0.f && l.y == 0.f &&
-                            l.z == 0.f && l.w == 0.f;
             float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
             float2 ax = make_float2(1.f, 0.f);
-            if (!bg) {
+            if (pixel_ray(P, px, py, f, l)) {
                 const int dt = s_dtype[wib];
-                if (dt == VRC_U8)
-                    res = march_ray<VRC_U8, COMP, SHADE, VRC_EE_ANALYTIC>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                else if (dt == VRC_U16)
-                    res = march_ray<VRC_U16, COMP, SHADE, VRC_EE_ANALYTIC>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                else res = march_ray<VRC_F32, COMP, SHADE, VRC_EE_ANALYTIC>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                if (P.L.B == 32) {
+                    if (dt == VRC_U8)
+                        res = march_ray<VRC_U8, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    else if (dt == VRC_U16)
+                        res = march_ray<VRC_U16, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    else
+                        res = march_ray<VRC_F32, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                } else {
+                    if (dt == VRC_U8)
+                        res = march_ray<VRC_U8, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    else if (dt == VRC_U16)
+                        res = march_ray<VRC_U16, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    else
+                        res = march_ray<VRC_F32, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                }
             }
             write_out(P, (size_t)py * P.W + px, res);
             if (P.aux) P.aux[(size_t)py * P.W + px] = ax;
+            flush_samples(cnt, state + 2);
         }
         __syncwarp();
         if (lane == 0) {

@@ -7,7 +7,7 @@ namespace {
 
 template <int DT, int COMP>
 cudaError_t launch_unshaded(const MarchParams& p, int, int num_sms, cudaStream_t s) {
-    return launch_ee<DT, COMP, VRC_SHADE_NONE>(p, num_sms, s);
+    return launch_pool<DT, COMP, VRC_SHADE_NONE>(p, num_sms, s);
 }
 
 template <int COMP>

@@ -135,6 +135,8 @@ vrc_status render_noalloc(const vrc_volume* vol, const vrc_tf* tf, const vrc_ren
     P.tf_width = tf->width;
     P.tf_lo = tf->lo;
     P.tf_hi = tf->hi;
+    P.tf_rcp = vrc::tf_reciprocal(tf->lo, tf->hi);
+    P.tf_wm1 = float(P.tf_width - 1);
     if (p->entry_exit_mode == VRC_EE_BUFFERS) {
         P.entry = reinterpret_cast<const float4*>(d_entry);
         P.exitp = reinterpret_cast<const float4*>(d_exit);

@@ -65,6 +65,8 @@ struct MarchParams {
     float spacing[3], spacing_rcp_half[3], vol_offset[3];
     float gscale[3];            // raw-value central difference -> gradient: 0.5/spacing * rwmScale / rangeMax
     float rwm_scale, rwm_offset, tf_lo, tf_hi;
+    float tf_rcp;               // RN(1 / (tf_hi - tf_lo)), 0 = divide (see tf_reciprocal)
+    float tf_wm1;               // tf_width - 1
     float step, ert;
     int use_ert;
     float iso;
@@ -121,6 +123,14 @@ constexpr int COMP_DVR_PREINT = 16;
 // (mod_compositing.frag:134); MIP / ISO / MOP / FHP / FHN use the TF alpha.
 inline bool alpha_corrected(int compositing, int classification) {
     return (compositing == VRC_DVR && classification == VRC_CLASSIFY_TF) || compositing == VRC_MIDA;
+}
+
+// RN(1 / (hi - lo)) for the march's corrected-product form of the TF
+// coordinate, or 0 where that form is not exact for every intensity (widths
+// outside [2^-60, 2^60]) and the march divides.
+inline float tf_reciprocal(float lo, float hi) {
+    const float b = hi - lo;
+    return b >= 0x1p-60f && b <= 0x1p60f ? 1.f / b : 0.f;
 }
 
 // One request of a batched launch.
