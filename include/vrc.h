@@ -328,7 +328,8 @@ typedef struct {
                                    holds the 2^3 level -- up to 2^30 cells -- else 4, also for batches;
                                    vrc_render_noalloc: the finest of 2, 4, 8 that fits its scratch), else 2,
                                    4, 8, 16 or the brick size */
-    int tile_width;             /* ray tile per warp: tile_width x (32 / tile_width) pixels; 0 = default (8) */
+    int tile_width;             /* ray tile per warp: tile_width x (32 / tile_width) pixels; 0 = default (8); frames
+                                   small enough to give each ray several lanes take tiles of their own */
     int region[4];              /* x, y, w, h of the pixel window to render; w or h 0 = the whole image */
     int classification;         /* vrc_classification, default VRC_CLASSIFY_TF */
     float mida_gamma;           /* "gammaValue" for VRC_MIDA, in [-1, 1], default 0 */
@@ -351,7 +352,7 @@ typedef struct {
     float kernel_ms;         /* device time of the march kernel on the context stream */
     float total_ms;          /* device time from first copy-in to last copy-out */
     int device_status;       /* 0, or an internal error code from the kernel */
-    int kernel_launches;     /* kernels this frame launched (occupancy levels + march) */
+    int kernel_launches;     /* kernels this frame launched (occupancy levels + march, one or two) */
 } vrc_render_stats;
 
 /* Render one frame.

@@ -218,7 +218,8 @@ vrc_status vrc_context_create(int device, vrc_context** out) {
             return VRC_ERR_CUDA;
         }
     }
-    if (cudaMalloc(&c->d_counters, 16 * sizeof(unsigned long long)) != cudaSuccess) {
+    if (cudaMalloc(&c->d_counters, 16 * sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMalloc(&c->d_queue, vrc::march_queue_bytes(c->num_sms)) != cudaSuccess) {
         vrc_context_destroy(c);
         return VRC_ERR_OUT_OF_MEMORY;
     }
@@ -239,6 +240,7 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_dist);
     cudaFree(c->d_dist_tmp);
     cudaFree(c->d_prefix);
+    cudaFree(c->d_queue);
     cudaFree(c->d_counters);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
@@ -1275,6 +1277,10 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
     P.counters = ctx->d_counters;
     P.status = reinterpret_cast<int*>(ctx->d_counters + 4);
     P.tile_counter = reinterpret_cast<unsigned int*>(ctx->d_counters + 5);
+    int march_launches = 0;
+    P.launches = &march_launches;
+    P.queue = reinterpret_cast<float4*>(ctx->d_queue);
+    P.queue_count = reinterpret_cast<unsigned int*>(ctx->d_counters + 6);
     VRC_CUDA(ctx, cudaEventRecord(ctx->ev[1], s));
     VRC_CUDA(ctx, vrc::launch_march(P, vol->desc.dtype, p->compositing, p->shading, ctx->num_sms, s));
     VRC_CUDA(ctx, cudaEventRecord(ctx->ev[2], s));
@@ -1289,7 +1295,7 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         stats->samples_shaded = double(h[2]);
         stats->skip_runs = double(h[3]);
         stats->device_status = int(h[4] & 0xffffffffu);
-        stats->kernel_launches = 1 + occ_launches;
+        stats->kernel_launches = march_launches + occ_launches;
         VRC_CUDA(ctx, cudaEventElapsedTime(&stats->kernel_ms, ctx->ev[1], ctx->ev[2]));
         VRC_CUDA(ctx, cudaEventElapsedTime(&stats->total_ms, ctx->ev[0], ctx->ev[3]));
         if (stats->device_status != 0) return fail(ctx, VRC_ERR_DEVICE, "vrc_render: kernel reported an error status");

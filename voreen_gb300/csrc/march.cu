@@ -62,6 +62,12 @@ __global__ void batch_begin_kernel(unsigned long long* state, int nreq) {
     if (threadIdx.x == 0) state[1] = global_ns();
 }
 
+template <int DT, int COMP, int SHADE, int BS>
+__device__ __forceinline__ void batch_ray(const MarchParams& P, float4 f, float4 l, int px, int py, RayState& st,
+                                          RayCounts& cnt) {
+    march_ray<DT, COMP, SHADE, BS, false, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, nullptr, st, cnt);
+}
+
 template <int COMP, int SHADE>
 __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS)
     march_batch_kernel(const BatchReq* __restrict__ reqs, int nreq, const unsigned* __restrict__ tile_prefix,
@@ -71,7 +77,8 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS)
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     MarchParams& P = s_par[wib];
     int cur = -1;
-    Counters cnt;
+    __shared__ WarpTotals totals[8];
+    if (lane == 0) totals[wib] = WarpTotals{};
     for (;;) {
         unsigned tile = 0;
         if (lane == 0) tile = atomicAdd(reinterpret_cast<unsigned*>(state), 1u);
@@ -98,41 +105,34 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS)
         const int tw = 1 << P.tile_wshift;
         const int px = P.rx0 + tx * tw + (lane & (tw - 1));
         const int py = P.ry0 + ty * (32 >> P.tile_wshift) + (lane >> P.tile_wshift);
+        RayState st;
+        st.begin(P);
+        RayCounts cnt;
         if (px < P.rx1 && py < P.ry1) {
             float4 f, l;
-            float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 ax = make_float2(1.f, 0.f);
+            if (P.aux) P.aux[(size_t)py * P.W + px] = make_float2(1.f, 0.f);
             if (pixel_ray(P, px, py, f, l)) {
                 const int dt = s_dtype[wib];
                 if (P.L.B == 32) {
-                    if (dt == VRC_U8)
-                        res = march_ray<VRC_U8, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                    else if (dt == VRC_U16)
-                        res = march_ray<VRC_U16, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                    else
-                        res = march_ray<VRC_F32, COMP, SHADE, 32, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    if (dt == VRC_U8) batch_ray<VRC_U8, COMP, SHADE, 32>(P, f, l, px, py, st, cnt);
+                    else if (dt == VRC_U16) batch_ray<VRC_U16, COMP, SHADE, 32>(P, f, l, px, py, st, cnt);
+                    else batch_ray<VRC_F32, COMP, SHADE, 32>(P, f, l, px, py, st, cnt);
                 } else {
-                    if (dt == VRC_U8)
-                        res = march_ray<VRC_U8, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                    else if (dt == VRC_U16)
-                        res = march_ray<VRC_U16, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
-                    else
-                        res = march_ray<VRC_F32, COMP, SHADE, 0, false>(P, P.tf_rgba8, P.tf_alpha, f, l, px, py, cnt, ax);
+                    if (dt == VRC_U8) batch_ray<VRC_U8, COMP, SHADE, 0>(P, f, l, px, py, st, cnt);
+                    else if (dt == VRC_U16) batch_ray<VRC_U16, COMP, SHADE, 0>(P, f, l, px, py, st, cnt);
+                    else batch_ray<VRC_F32, COMP, SHADE, 0>(P, f, l, px, py, st, cnt);
                 }
             }
-            write_out(P, (size_t)py * P.W + px, res);
-            if (P.aux) P.aux[(size_t)py * P.W + px] = ax;
-            flush_samples(cnt, state + 2);
+            write_out(P, (size_t)py * P.W + px, st.res);
         }
+        add_tile(totals[wib], st.loop, cnt);
         __syncwarp();
         if (lane == 0) {
             __threadfence();
             atomicMax(state + 3 + r, global_ns());
         }
     }
-    unsigned long long a = cnt.samples;
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(FULL, a, o);
-    if (lane == 0) atomicAdd(state + 2, a);
+    if (lane == 0) atomicAdd(state + 2, totals[wib].samples);
 }
 
 template <int COMP, int SHADE>

@@ -5,7 +5,9 @@
 // Design:
 //  * persistent grid (a few CTAs per SM); each warp pulls 8x4 ray tiles from
 //    a global counter, so a warp's 32 rays are adjacent on screen and walk
-//    the same bricks;
+//    the same bricks. Small frames give each ray 2 to 8 lanes, and larger ones
+//    hand the rays left over when the tiles run out to a second kernel with 8
+//    lanes a ray (launch_t has the rule and the figures);
 //  * the transfer function sits in shared memory as its RGBA8 entries plus
 //    a table of 256 alphas (one per alpha byte) that already carry the
 //    opacity correction 1-(1-a)^(step*200), computed on the host with the
@@ -29,9 +31,9 @@
 //    instead of a division, one distance byte decides emptiness, the box exit
 //    is two FMAs an axis on per-ray constants. Together, us per frame before
 //    and after (bits unchanged): 512^3 u16 shaded DVR at 1080p 678 -> 475, its
-//    MIP 830 -> 690, pre-integrated 854 -> 656, 2048x2048x1024 tubes at 4K
-//    21,600 -> 16,550, 64 mixed requests 15,090 -> 10,900, 64^3 u8 at 256^2
-//    111 -> 85;
+//    MIP 830 -> 661, pre-integrated 854 -> 605, 2048x2048x1024 tubes at 4K
+//    21,600 -> 15,440, 64 mixed requests 15,090 -> 11,030; with the lanes a
+//    ray, shaded DVR 475 -> 389, 64^3 u8 at 256^2 111 -> 54;
 //  * gradients (central differences, mod_gradients.frag:202-214) are six
 //    lookups at +-1/dim in texture space, clamped like the intensity sample
 //    and read from the centre's brick apron (another brick only when rounding
@@ -75,7 +77,8 @@ __device__ __forceinline__ float small_uint_to_float(unsigned v) {
     return __fsub_rn(__int_as_float(0x4B000000u | v), 8388608.f);
 }
 // Pairs of FP32 in one 64-bit register pair: add / mul / fma of both halves
-// in one issue slot, each half rounded as the scalar instruction rounds it.
+// in one issue slot, each half rounded as the scalar instruction rounds it
+// (never a product that an addition follows: a pair of those came out fused).
 // The march is bound by instruction issue and load latency, so the sample's
 // eight normalisations and products and the gradient's lerps run on pairs.
 using f2 = unsigned long long;
@@ -490,12 +493,32 @@ __device__ __forceinline__ void write_out(const MarchParams& P, size_t pix, floa
     }
 }
 
-// Per thread. A frame has at most 2^28 rays of 255^2 samples; flush_samples
-// (after each tile) keeps the 32-bit counts of a thread that marches many of
-// them from running over.
-struct Counters {
-    unsigned samples = 0, fetched = 0, shaded = 0, runs = 0;
+// Samples of one ray by what became of them, two counts of at most 255^2 to a
+// register: fetched in the low half, shaded in the high half; skip runs in the
+// low half, pre-integration's reads of a skipped previous sample (fetched
+// samples too) in the high half.
+struct RayCounts {
+    unsigned fetched_shaded = 0, runs = 0;
 };
+
+// Adds a tile's rays to the warp's totals in shared memory: the totals take no
+// registers while a ray marches. `loop`: the samples of this lane's ray.
+struct WarpTotals {
+    unsigned long long samples, fetched, shaded, runs;
+};
+__device__ __forceinline__ void add_tile(WarpTotals& w, int loop, const RayCounts& c) {
+    // at most 32 x 2 x 255^2 each
+    const unsigned a = __reduce_add_sync(FULL, (unsigned)loop);
+    const unsigned b = __reduce_add_sync(FULL, (c.fetched_shaded & 0xffffu) + (c.runs >> 16));
+    const unsigned d = __reduce_add_sync(FULL, c.fetched_shaded >> 16);
+    const unsigned e = __reduce_add_sync(FULL, c.runs & 0xffffu);
+    if ((threadIdx.x & 31) == 0) {
+        w.samples += a;
+        w.fetched += b;
+        w.shaded += d;
+        w.runs += e;
+    }
+}
 
 // MIP: true when no sample of a cell whose largest normalised value is `m`
 // can exceed the ray's maximum real-world intensity `max_int`, so the cell
@@ -534,37 +557,18 @@ __device__ __forceinline__ float cell_exit_t(const MarchParams& P, float4 f, flo
     return tmax;
 }
 
-// The same for a box of cells [c - r, c + r] on each axis, clipped to the
-// grid (a face on the grid's border is never left).
-__device__ __noinline__ float box_exit_t(const MarchParams& P, float4 f, float dx, float dy, float dz, int cx, int cy,
-                                         int cz, int r) {
-    const int C = 1 << P.cshift;
-    const float fo[3] = {f.x, f.y, f.z}, di[3] = {dx, dy, dz};
-    const int ci[3] = {cx, cy, cz};
-    float tmax = INFINITY;
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        const float a = P.dimf[i] * fo[i] - 0.5f, b = P.dimf[i] * di[i];
-        if (b > 0.f && ci[i] + r < P.nc[i] - 1) {
-            tmax = fminf(tmax, __fdividef((float)((ci[i] + r + 1) * C) - P.skip_margin - a, b));
-        } else if (b < 0.f && ci[i] - r > 0) {
-            tmax = fminf(tmax, __fdividef((float)((ci[i] - r) * C) + P.skip_margin - a, b));
-        }
-    }
-    return tmax;
-}
-
-// box_exit_t with the ray's part computed once: along an axis with voxel
-// position a + t * b the box of cells [c - r, c + r] of edge C is left at
+// The same for a box of cells [c - r, c + r] on each axis, the ray's part
+// computed once: an axis with voxel position a + t * b is left at
 //   b > 0:  ((c + r + 1) * C - margin - a) / b = c * C/b + r * C/b + (C - margin - a)/b
 //   b < 0:  ((c - r) * C + margin - a) / b     = c * C/b - r * C/b + (margin - a)/b,
 // two FMAs on per-ray constants. Each term is below the volume's edge in
 // voxels, so FP32 rounding moves the face by less than 4 * 2^-23 of that
 // edge; the margin is 0.01 + 2e-5 of it. An axis the ray does not move along
 // gives infinities or NaN, which fminf drops where they mean "never left".
-// Faces on the grid's border count like others: the far ones lie beyond every
-// sample, the near ones would cost a ray outside them single steps (the
-// caller falls back to box_exit_t where a box at the border gives no advance).
+// A face on the grid's border is never left (samples beyond it clamp to the
+// border cells): at() counts it like others, which costs samples within the
+// volume nothing but the last half voxel at a near face; border() drops it and
+// is taken where at() gives a ray no advance.
 struct BoxExit {
     float k1[3], k0[3];
     __device__ __forceinline__ void set(const MarchParams& P, float4 f, float dx, float dy, float dz) {
@@ -583,6 +587,16 @@ struct BoxExit {
         const float ty = __fmaf_rn((float)cy, k1[1], __fmaf_rn(fr, fabsf(k1[1]), k0[1]));
         const float tz = __fmaf_rn((float)cz, k1[2], __fmaf_rn(fr, fabsf(k1[2]), k0[2]));
         return fminf(fminf(tx, ty), tz);
+    }
+    __device__ __forceinline__ float border(const MarchParams& P, int cx, int cy, int cz, int r) const {
+        const float fr = (float)r;
+        const int c[3] = {cx, cy, cz};
+        float t = INFINITY;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (k1[i] > 0.f ? c[i] + r < P.nc[i] - 1 : c[i] - r > 0)
+                t = fminf(t, __fmaf_rn((float)c[i], k1[i], __fmaf_rn(fr, fabsf(k1[i]), k0[i])));
+        return t;
     }
 };
 
@@ -761,20 +775,23 @@ __device__ __forceinline__ F3 central_gradient(const MarchParams& P, const typen
     // v<axis><side> pairs over z (0, 1); the z sides as the pair (-1, 2)
 #define VRC_Z(X, Y) V::raw2(__ldg(vox + (X) + (Y) * S), __ldg(vox + (X) + (Y) * S + S2))
 #define VRC_E(X, Y) V::raw2(__ldg(vox + (X) + (Y) * S - S2), __ldg(vox + (X) + (Y) * S + 2 * S2))
+    const f2 fx2 = pk(fx, fx), fy2 = pk(fy, fy);
+    const float gxp = vxp - fxp, gxm = vxm - fxm, gyp = vyp - fyp, gym = vym - fym;
     const f2 xm0 = VRC_Z(-1, 0), xm1 = VRC_Z(-1, 1), xp0 = VRC_Z(2, 0), xp1 = VRC_Z(2, 1);
     const f2 ym0 = VRC_Z(0, -1), ym1 = VRC_Z(1, -1), yp0 = VRC_Z(0, 2), yp1 = VRC_Z(1, 2);
-    const f2 z00 = VRC_E(0, 0), z10 = VRC_E(1, 0), z01 = VRC_E(0, 1), z11 = VRC_E(1, 1);
-#undef VRC_Z
-#undef VRC_E
-    const f2 fx2 = pk(fx, fx), fy2 = pk(fy, fy);
-    const f2 e0 = lerp2(fx2, c.c00, c.c10), e1 = lerp2(fx2, c.c01, c.c11);  // the sample's rows at y = 0, 1
-    const f2 f = lerp2(fy2, e0, e1);                                          // ... at z = 0, 1
-    const f2 z = lerp2(fy2, lerp2(fx2, z00, z10), lerp2(fx2, z01, z11));      // the same at z = -1, 2
-    const float gxp = vxp - fxp, gxm = vxm - fxm, gyp = vyp - fyp, gym = vym - fym;
     const f2 xp = lerp2(fy2, lerp2(pk(gxp, gxp), c.c10, xp0), lerp2(pk(gxp, gxp), c.c11, xp1));
     const f2 xm = lerp2(fy2, lerp2(pk(gxm, gxm), xm0, c.c00), lerp2(pk(gxm, gxm), xm1, c.c01));
+    const f2 e0 = lerp2(fx2, c.c00, c.c10), e1 = lerp2(fx2, c.c01, c.c11);
     const f2 yp = lerp2(pk(gyp, gyp), e1, lerp2(fx2, yp0, yp1));
     const f2 ym = lerp2(pk(gym, gym), lerp2(fx2, ym0, ym1), e0);
+    // the z sides after the others: 24 loads in flight at once cost the 80
+    // registers spills (512^3 tubes 16.2 ms a 4K frame against 15.4)
+    asm volatile("" ::: "memory");
+    const f2 z00 = VRC_E(0, 0), z10 = VRC_E(1, 0), z01 = VRC_E(0, 1), z11 = VRC_E(1, 1);
+    const f2 f = lerp2(fy2, e0, e1);
+    const f2 z = lerp2(fy2, lerp2(fx2, z00, z10), lerp2(fx2, z01, z11));
+#undef VRC_Z
+#undef VRC_E
     const float v0 = __fmaf_rn(fz, hi2(xp) - lo2(xp), lo2(xp)), v3 = __fmaf_rn(fz, hi2(xm) - lo2(xm), lo2(xm));
     const float v1 = __fmaf_rn(fz, hi2(yp) - lo2(yp), lo2(yp)), v4 = __fmaf_rn(fz, hi2(ym) - lo2(ym), lo2(ym));
     const float v2 = __fmaf_rn(vzp - fzp, hi2(z) - hi2(f), hi2(f)), v5 = __fmaf_rn(vzm - fzm, lo2(f) - lo2(z), lo2(z));
@@ -835,6 +852,13 @@ __device__ __forceinline__ void composite(const MarchParams& P, float4& res, flo
     }
 }
 
+// The auxiliary output of a pixel whose first sample with alpha > 0 lies at t
+// with squared gradient magnitude g2 (no such sample: (1, 0), written with the
+// pixel before its ray marches).
+__device__ __forceinline__ void write_aux(const MarchParams& P, int px, int py, float t, float tend, float g2) {
+    P.aux[(size_t)py * P.W + px] = make_float2(__fdividef(t, fmaxf(tend, 1e-20f)), sqrtf(g2) * P.aux_gscale);
+}
+
 // Ray direction and end (cpuraycaster.cpp:216-232); degenerate rays take one sample.
 __device__ __forceinline__ float ray_setup(const MarchParams& P, float4 f, float4 l, float& dx, float& dy, float& dz) {
     dx = s_(l.x, f.x);
@@ -857,7 +881,8 @@ __device__ __forceinline__ float ray_setup(const MarchParams& P, float4 f, float
 __device__ __forceinline__ float4 tf_colour(const MarchParams& P, const uchar4* __restrict__ s_tf,
                                             const float* __restrict__ s_alpha, float rw) {
     const uchar4 e8 = s_tf[(int)a_(m_(rw_to_tf(rw, P.tf_lo, P.tf_hi, P.tf_rcp), P.tf_wm1), 0.5f)];
-    return make_float4(Vox<VRC_U8>::norm(e8.x), Vox<VRC_U8>::norm(e8.y), Vox<VRC_U8>::norm(e8.z), s_alpha[e8.w]);
+    const f2 rg = Vox<VRC_U8>::norm2(Vox<VRC_U8>::raw2(e8.x, e8.y));
+    return make_float4(lo2(rg), hi2(rg), Vox<VRC_U8>::norm(e8.z), s_alpha[e8.w]);
 }
 
 // The empty-space test of one sample: whether its cell is empty for the ray
@@ -885,9 +910,7 @@ __device__ __forceinline__ bool empty_cell(const MarchParams& P, const BoxExit& 
         if (tf_empty) {
             const int r = d - 1;
             tsafe = bx.at(fcx, fcy, fcz, r);
-            if (!(tsafe > t) && (fcx <= r || fcy <= r || fcz <= r || fcx + r >= P.nc[0] - 1 ||
-                                 fcy + r >= P.nc[1] - 1 || fcz + r >= P.nc[2] - 1))
-                tsafe = box_exit_t(P, f, dx, dy, dz, fcx, fcy, fcz, r);
+            if (!(tsafe > t)) tsafe = bx.border(P, fcx, fcy, fcz, r);
             return true;
         }
         if (!mip_skip) return false;
@@ -910,12 +933,41 @@ __device__ __forceinline__ bool empty_cell(const MarchParams& P, const BoxExit& 
     return true;
 }
 
+// What a ray's samples so far have left; t, loop: the next sample. In the
+// queue of unfinished rays: two float4.
+struct RayState {
+    float4 res;
+    float max_int, t;
+    int loop;
+    bool hit;  // the auxiliary output has the first sample with alpha > 0
+    __device__ __forceinline__ void begin(const MarchParams& P) {
+        res = make_float4(0.f, 0.f, 0.f, 0.f);
+        max_int = t = 0.f;
+        loop = 0;
+        hit = P.aux == nullptr;
+    }
+    __device__ __forceinline__ void store(float4* q, int pix) const {
+        q[0] = res;
+        q[1] = make_float4(max_int, t, __int_as_float(loop | (hit ? 1 << 30 : 0)), __int_as_float(pix));
+    }
+    __device__ __forceinline__ int load(const float4* q) {
+        res = q[0];
+        const float4 r = q[1];
+        max_int = r.x;
+        t = r.y;
+        loop = __float_as_int(r.z) & ((1 << 30) - 1);
+        hit = (__float_as_int(r.z) >> 30) != 0;
+        return __float_as_int(r.w);
+    }
+};
+
 // One ray on one thread: the loop of cpuraycaster.cpp:239-317 with the GLSL
-// compositing.
-template <int DT, int COMP, int SHADE, int BS, bool POOL>
-__device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* __restrict__ s_tf,
-                                            const float* __restrict__ s_alpha, float4 f, float4 l, int px, int py,
-                                            Counters& cnt, float2& aux) {
+// compositing. STOP: the ray is left unfinished (false) a sample or run after
+// *stop becomes set.
+template <int DT, int COMP, int SHADE, int BS, bool POOL, bool STOP>
+__device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __restrict__ s_tf,
+                                          const float* __restrict__ s_alpha, float4 f, float4 l, int px, int py,
+                                          const volatile int* stop, RayState& st, RayCounts& cnt) {
     using T = typename Vox<DT>::T;
     using G = BrickGeom<BS>;
     const T* __restrict__ bricks = reinterpret_cast<const T*>(P.bricks);
@@ -928,23 +980,29 @@ __device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* 
     constexpr bool ERT = !(COMP == VRC_MIP || COMP == VRC_MOP || COMP == VRC_MIDA);
     BoxExit bx;
     bx.set(P, f, dx, dy, dz);
-    float4 res = make_float4(0.f, 0.f, 0.f, 0.f);
-    float max_int = 0.f;
+    float4& res = st.res;
+    float &max_int = st.max_int, &t = st.t;
+    int& loop = st.loop;
+    bool& hit = st.hit;
+    st.begin(P);
     float last = 0.f;  // lastIntensity (cpuraycaster.cpp:235), TF-normalised
     // pre-integration: whether the previous sample lay in an empty cell, and
     // whether `last` still has to be read at t_last (the last skipped sample)
     bool prev_empty = false, last_stale = false;
     float t_last = 0.f;
-    float t = 0.f;
-    float hit_t = -1.f, hit_g = 0.f;  // first sample with alpha > 0 (auxiliary output)
     long long marked = -1;             // last brick recorded as read (cache refinement)
     // POOL: the brick of the last fetched sample and its start (a slot lookup
     // each); a device-resident pool's address is two multiply-adds
     int cached_brick = -1;
     const T* cached_base = nullptr;
     bool finished = false;
-    int loop = 0;
+    int stopped = 0;
     while (!finished && loop < LOOP_CAP) {
+        // read for the next pass: the load's latency stays off the chain
+        if (STOP) {
+            if (stopped) return false;
+            stopped = *stop;
+        }
         SamplePos p;
         p.set(P, f, dx, dy, dz, t);
         bool skip_after = false;  // pre-integration: skip the samples after this one in its empty cell
@@ -1011,7 +1069,7 @@ __device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* 
             } else {
                 b = bricks + (long long)brick * G::stride(P.L);
             }
-            ++cnt.fetched;
+            ++cnt.fetched_shaded;
             const float fx = s_(p.vx, p.flx), fy = s_(p.vy, p.fly), fz = s_(p.vz, p.flz);
             const int S = G::S(P.L);
             const int o = ((p.iz - (bZ << sh) + APRON_LO) * S + (p.iy - (bY << sh) + APRON_LO)) * S +
@@ -1030,7 +1088,7 @@ __device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* 
             float4 c;
             if (PI) {
                 if (last_stale) {  // the previous sample was skipped: read its TF coordinate
-                    ++cnt.fetched;
+                    cnt.runs += 0x10000u;
                     const float px_ = a_(f.x, m_(t_last, dx)), py_ = a_(f.y, m_(t_last, dy)),
                                 pz_ = a_(f.z, m_(t_last, dz));
                     const float rwp = a_(m_(tap_norm<DT, POOL>(P, bricks, to_voxel(P, 0, px_), to_voxel(P, 1, py_),
@@ -1049,14 +1107,18 @@ __device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* 
                 c = tf_colour(P, s_tf, s_alpha, rw);
             }
             if (c.w > 0.f) {
+                float gmag2 = 0.f;
                 if (SHADE == VRC_SHADE_PHONG) {
-                    ++cnt.shaded;
+                    cnt.fetched_shaded += 0x10000u;
                     const F3 g = t == 0.f ? clip_border_gradient(P, F3{p.sx, p.sy, p.sz}, F3{dx, dy, dz}, px, py)
                                           : central_gradient<DT, BS, POOL>(P, bricks, b, vox, raw, p, fx, fy, fz);
-                    if (hit_t < 0.f) hit_g = sqrtf(g.x * g.x + g.y * g.y + g.z * g.z);
+                    if (!hit) gmag2 = g.x * g.x + g.y * g.y + g.z * g.z;
                     shade(P, p, g, c);
                 }
-                if (hit_t < 0.f) hit_t = t;
+                if (!hit) {
+                    hit = true;
+                    write_aux(P, px, py, t, tend, gmag2);
+                }
                 if (COMP == VRC_FHP) {
                     c = make_float4(p.sx, p.sy, p.sz, 1.f);  // texture-space position
                 } else if (COMP == VRC_FHN) {
@@ -1103,9 +1165,118 @@ __device__ __forceinline__ float4 march_ray(const MarchParams& P, const uchar4* 
             }
         }
     }
-    cnt.samples += (unsigned)loop;
-    aux = hit_t < 0.f ? make_float2(1.f, 0.f) : make_float2(__fdividef(hit_t, fmaxf(tend, 1e-20f)), hit_g * P.aux_gscale);
-    return res;
+    return true;
+}
+
+// One ray on G neighbouring lanes: lane k of the group takes the k-th of the
+// next G samples, and the group then composites them in order, every lane the
+// same (lane 0's result is the ray's). All lanes of the warp call it together;
+// `alive` is the same in a group, and so are f, l, px, py. A ray's chain of
+// dependent loads gets G times shorter where its samples are occupied, for G
+// times the lanes on a run through empty space.
+template <int DT, int COMP, int SHADE, int BS, int G>
+__device__ __forceinline__ void march_ray_group(const MarchParams& P, const uchar4* __restrict__ s_tf,
+                                                const float* __restrict__ s_alpha, bool alive, float4 f, float4 l,
+                                                int px, int py, RayState& st, RayCounts& cnt) {
+    using T = typename Vox<DT>::T;
+    using BG = BrickGeom<BS>;
+    constexpr bool ERT = !(COMP == VRC_MIP || COMP == VRC_MOP || COMP == VRC_MIDA);
+    constexpr unsigned GM = (1u << G) - 1u;
+    const T* __restrict__ bricks = reinterpret_cast<const T*>(P.bricks);
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1), base = lane & ~(G - 1);
+    const float step = P.step;
+    float dx, dy, dz;
+    const float tend = ray_setup(P, f, l, dx, dy, dz);
+    BoxExit bx;
+    bx.set(P, f, dx, dy, dz);
+    float4& res = st.res;
+    float &max_int = st.max_int, &t = st.t;
+    int& loop = st.loop;
+    bool& hit = st.hit;
+    bool finished = !alive;
+    while (__any_sync(FULL, !finished)) {
+        // this lane's sample: t advanced `sub` times, as the one-at-a-time loop does
+        float tl = t, tn = t;
+#pragma unroll
+        for (int k = 1; k < G; ++k) {
+            tn = a_(tn, step);
+            if (k == sub) tl = tn;
+        }
+        tn = a_(tn, step);
+        const bool valid = !finished && loop + sub < LOOP_CAP && (sub == 0 || !(tl > tend));
+        float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+        float rw = 0.f, tsafe = 0.f, gmag2 = 0.f;
+        bool empty = false;
+        if (valid) {
+            SamplePos p;
+            p.set(P, f, dx, dy, dz, tl);
+            if (P.occupancy) empty = empty_cell<COMP>(P, bx, f, dx, dy, dz, p, tl, max_int, tsafe);
+            if (!empty) {
+                const int sh = BG::shift(P.L), S = BG::S(P.L);
+                const int bX = p.ix >> sh, bY = p.iy >> sh, bZ = p.iz >> sh;
+                const T* __restrict__ b =
+                    bricks + (long long)((bZ * P.L.nb[1] + bY) * P.L.nb[0] + bX) * BG::stride(P.L);
+                const float fx = s_(p.vx, p.flx), fy = s_(p.vy, p.fly), fz = s_(p.vz, p.flz);
+                const T* __restrict__ vox = b + ((p.iz - (bZ << sh) + APRON_LO) * S + (p.iy - (bY << sh) + APRON_LO)) * S +
+                                            (p.ix - (bX << sh) + APRON_LO);
+                const Raw8 raw = load8<DT>(vox, S, BG::S2(P.L));
+                rw = a_(m_(tri8<DT>(raw, fx, fy, fz), P.rwm_scale), P.rwm_offset);
+                c = tf_colour(P, s_tf, s_alpha, rw);
+                if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) {
+                    const F3 g = tl == 0.f ? clip_border_gradient(P, F3{p.sx, p.sy, p.sz}, F3{dx, dy, dz}, px, py)
+                                           : central_gradient<DT, BS, false>(P, bricks, b, vox, raw, p, fx, fy, fz);
+                    if (!hit) gmag2 = g.x * g.x + g.y * g.y + g.z * g.z;
+                    shade(P, p, g, c);
+                }
+            }
+        }
+        const unsigned val = __ballot_sync(FULL, valid), emp = __ballot_sync(FULL, empty);
+        const unsigned vis = __ballot_sync(FULL, c.w > 0.f);
+        const unsigned gval = (val >> base) & GM, gfet = gval & ~(emp >> base), gvis = (vis >> base) & GM;
+        int used = __popc(gval);  // samples of this pass that the ray takes
+        bool stop = false;
+        if (vis != 0u || (ERT && P.ert <= 0.f)) {
+            if (!hit && gvis) {
+                hit = true;
+                if (sub == __ffs(gvis) - 1) write_aux(P, px, py, tl, tend, gmag2);
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                const float4 ck = make_float4(__shfl_sync(FULL, c.x, k, G), __shfl_sync(FULL, c.y, k, G),
+                                              __shfl_sync(FULL, c.z, k, G), __shfl_sync(FULL, c.w, k, G));
+                const float rk = COMP == VRC_MIP || COMP == VRC_MIDA ? __shfl_sync(FULL, rw, k, G) : 0.f;
+                if (!stop && ((gfet >> k) & 1u)) {
+                    if ((gvis >> k) & 1u) composite<COMP>(P, res, max_int, ck, rk);
+                    if (ERT && res.w >= P.ert) {
+                        res.w = 1.f;
+                        stop = true;
+                        used = k + 1;
+                    }
+                }
+            }
+        }
+        if (sub < used && ((gfet >> sub) & 1u)) {
+            ++cnt.fetched_shaded;
+            if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) cnt.fetched_shaded += 0x10000u;
+        }
+        loop += used;
+        finished = finished || stop || used < G || tn > tend || loop >= LOOP_CAP;
+        t = tn;
+        const float ts = __shfl_sync(FULL, tsafe, G - 1, G);
+        if (!finished && ((emp >> (base + G - 1)) & 1u)) {
+            // the last sample's cell is empty: so are the samples up to its exit
+            if (sub == 0) ++cnt.runs;
+            const float lim = fminf(ts, tend);
+            while (t <= lim && loop < LOOP_CAP) {
+                jump_empty_run(t, loop, step, lim);
+                if (t <= lim && loop < LOOP_CAP) {
+                    t = a_(t, step);
+                    ++loop;
+                }
+            }
+            finished = t > tend || loop >= LOOP_CAP;
+        }
+    }
 }
 
 // The TF in shared memory: 256 alphas, then the RGBA8 entries (17 KB at 4096
@@ -1132,43 +1303,35 @@ __device__ __forceinline__ bool pixel_ray(const MarchParams& P, int px, int py, 
              l.w == 0.f);
 }
 
-// A tile adds at most 255^2 samples to a thread.
-__device__ __forceinline__ void flush_samples(Counters& cnt, unsigned long long* samples) {
-    if (cnt.samples < 0x80000000u) return;
-    atomicAdd(samples, (unsigned long long)cnt.samples);
-    cnt.samples = 0;
-}
-
-__device__ __forceinline__ void add_counters(const MarchParams& P, const Counters& cnt) {
-    if (!P.counters) return;
-    unsigned long long a = cnt.samples, b = cnt.fetched, c = cnt.shaded, d = cnt.runs;
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(FULL, a, o);
-        b += __shfl_xor_sync(FULL, b, o);
-        c += __shfl_xor_sync(FULL, c, o);
-        d += __shfl_xor_sync(FULL, d, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(P.counters + 0, a);
-        atomicAdd(P.counters + 1, b);
-        atomicAdd(P.counters + 2, c);
-        atomicAdd(P.counters + 3, d);
-    }
+__device__ __forceinline__ void add_counters(const MarchParams& P, const WarpTotals& w) {
+    if (!P.counters || (threadIdx.x & 31) != 0) return;
+    atomicAdd(P.counters + 0, w.samples);
+    atomicAdd(P.counters + 1, w.fetched);
+    atomicAdd(P.counters + 2, w.shaded);
+    atomicAdd(P.counters + 3, w.runs);
 }
 
 #ifndef VRC_MARCH_MIN_BLOCKS
 #define VRC_MARCH_MIN_BLOCKS 3
 #endif
 
-template <int DT, int COMP, int SHADE, int BS, bool POOL>
+// One ray per lane. QUEUE: when the tiles run out, the warps of a CTA leave
+// their unfinished rays to march_queue_kernel: the longest rays of a frame
+// (those that graze a shell, the whole of a MIP) take as long on one lane each
+// as a tenth of the pixels do, so the frame would end on a few slow warps.
+template <int DT, int COMP, int SHADE, int BS, bool POOL, bool QUEUE>
 __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_kernel(const __grid_constant__ MarchParams P) {
     extern __shared__ float4 s_raw[];
     float* s_alpha = reinterpret_cast<float*>(s_raw);
     uchar4* s_tf = reinterpret_cast<uchar4*>(s_alpha + 256);
+    __shared__ WarpTotals totals[8];
+    __shared__ int s_stop;
+    if (threadIdx.x == 0) s_stop = 0;
     stage_tf(P, s_alpha, s_tf);
     const int lane = threadIdx.x & 31;
     const int ntiles = P.tiles_x * P.tiles_y;
-    Counters cnt;
+    WarpTotals& mine = totals[threadIdx.x >> 5];
+    if (lane == 0) mine = WarpTotals{};
     for (;;) {
         int tile = 0;
         if (lane == 0) tile = (int)atomicAdd(P.tile_counter, 1u);
@@ -1178,19 +1341,85 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_kernel(const 
         const int tw = 1 << P.tile_wshift;
         const int px = P.rx0 + tx * tw + (lane & (tw - 1));
         const int py = P.ry0 + ty * (32 >> P.tile_wshift) + (lane >> P.tile_wshift);
+        RayState st;
+        st.begin(P);
+        RayCounts cnt;
+        bool done = true;
+        const size_t pix = (size_t)py * P.W + px;
         if (px < P.rx1 && py < P.ry1) {
-            const size_t pix = (size_t)py * P.W + px;
+            if (P.aux) P.aux[pix] = make_float2(1.f, 0.f);
             float4 f, l;
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-            float2 ax = make_float2(1.f, 0.f);
             if (pixel_ray(P, px, py, f, l))
-                r = march_ray<DT, COMP, SHADE, BS, POOL>(P, s_tf, s_alpha, f, l, px, py, cnt, ax);
-            write_out(P, pix, r);
-            if (P.aux) P.aux[pix] = ax;
-            if (P.counters) flush_samples(cnt, P.counters);
+                done = march_ray<DT, COMP, SHADE, BS, POOL, QUEUE>(P, s_tf, s_alpha, f, l, px, py, &s_stop, st, cnt);
+            if (done) write_out(P, pix, st.res);
+        }
+        add_tile(mine, done ? st.loop : 0, cnt);
+        if (QUEUE) {
+            const unsigned left = __ballot_sync(FULL, !done);
+            if (left) {
+                unsigned at = 0;
+                if (lane == 0) at = atomicAdd(P.queue_count, (unsigned)__popc(left));
+                at = __shfl_sync(FULL, at, 0) + __popc(left & ((1u << lane) - 1u));
+                if (!done) st.store(P.queue + 2 * (size_t)at, (int)pix);
+            }
         }
     }
-    add_counters(P, cnt);
+    if (QUEUE && lane == 0) *const_cast<volatile int*>(&s_stop) = 1;
+    add_counters(P, mine);
+}
+
+// G lanes per ray, a warp takes 32 / G pixels: tiles of the frame, or the
+// queue march_kernel left.
+template <int G> struct GroupTile {
+    static constexpr int W = G == 8 ? 2 : 4, H = 32 / G / W;
+};
+template <int DT, int COMP, int SHADE, int BS, int G, bool QUEUE>
+__global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_group_kernel(const __grid_constant__ MarchParams P) {
+    extern __shared__ float4 s_raw[];
+    float* s_alpha = reinterpret_cast<float*>(s_raw);
+    uchar4* s_tf = reinterpret_cast<uchar4*>(s_alpha + 256);
+    const int lane = threadIdx.x & 31, ray = lane / G;
+    const unsigned queued = QUEUE ? *P.queue_count : 0u;
+    const int ntiles = QUEUE ? (int)((queued + 32 / G - 1) / (32 / G)) : P.tiles_x * P.tiles_y;
+    if (QUEUE && (int)blockIdx.x * 8 >= ntiles) return;
+    stage_tf(P, s_alpha, s_tf);
+    __shared__ WarpTotals totals[8];
+    WarpTotals& mine = totals[threadIdx.x >> 5];
+    if (lane == 0) mine = WarpTotals{};
+    for (;;) {
+        int tile = 0;
+        if (lane == 0) tile = (int)atomicAdd(QUEUE ? P.queue_count + 1 : P.tile_counter, 1u);
+        tile = __shfl_sync(FULL, tile, 0);
+        if (tile >= ntiles) break;
+        RayState st;
+        st.begin(P);
+        int px, py;
+        bool inside;
+        if (QUEUE) {
+            const unsigned q = (unsigned)tile * (32 / G) + ray;
+            inside = q < queued;
+            const int pix = inside ? st.load(P.queue + 2 * (size_t)q) : 0;
+            py = pix / P.W;
+            px = pix - py * P.W;
+        } else {
+            px = P.rx0 + (tile % P.tiles_x) * GroupTile<G>::W + ray % GroupTile<G>::W;
+            py = P.ry0 + (tile / P.tiles_x) * GroupTile<G>::H + ray / GroupTile<G>::W;
+            inside = px < P.rx1 && py < P.ry1;
+        }
+        const size_t pix = (size_t)py * P.W + px;
+        const bool writes = inside && (lane & (G - 1)) == 0;
+        if (!QUEUE && writes && P.aux) P.aux[pix] = make_float2(1.f, 0.f);
+        __syncwarp();  // before any lane of the group writes the pixel's first hit
+        float4 f = make_float4(0.f, 0.f, 0.f, 0.f), l = f;
+        const bool alive = inside && pixel_ray(P, px, py, f, l);
+        if (__any_sync(FULL, alive)) {
+            RayCounts cnt;
+            march_ray_group<DT, COMP, SHADE, BS, G>(P, s_tf, s_alpha, alive, f, l, px, py, st, cnt);
+            add_tile(mine, writes ? st.loop : 0, cnt);
+        }
+        if (writes) write_out(P, pix, st.res);
+    }
+    add_counters(P, mine);
 }
 
 // Resident CTAs per SM of one kernel for a dynamic shared memory size,
@@ -1244,20 +1473,76 @@ cudaError_t resident_ctas(K k, size_t smem, int* per_sm) {
     return cudaSuccess;
 }
 
-template <int DT, int COMP, int SHADE, int BS, bool POOL>
-cudaError_t launch_t(const MarchParams& p, int num_sms, cudaStream_t s) {
-    auto k = march_kernel<DT, COMP, SHADE, BS, POOL>;
-    const size_t smem = 256 * sizeof(float) + (size_t)p.tf_width * sizeof(uchar4);
+inline size_t tf_smem(const MarchParams& p) { return 256 * sizeof(float) + (size_t)p.tf_width * sizeof(uchar4); }
+
+// Persistent launch: as many CTAs as are resident at once, or as 8 warps a
+// CTA need for the tiles.
+template <typename K>
+cudaError_t launch_persistent(K k, const MarchParams& p, long long tiles, int num_sms, cudaStream_t s) {
     int per_sm = 0;
-    cudaError_t e = resident_ctas(k, smem, &per_sm);
+    cudaError_t e = resident_ctas(k, tf_smem(p), &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
-    const long long tiles = (long long)p.tiles_x * p.tiles_y;
     long long grid = (long long)num_sms * per_sm;
-    const long long need = (tiles + 7) / 8;  // 8 warps per CTA
+    const long long need = (tiles + 7) / 8;
     if (grid > need) grid = need < 1 ? 1 : need;
-    k<<<(unsigned)grid, 256, smem, s>>>(p);
+    k<<<(unsigned)grid, 256, tf_smem(p), s>>>(p);
+    if (p.launches) ++*p.launches;
     return cudaGetLastError();
+}
+
+template <int DT, int COMP, int SHADE, int BS, int G>
+cudaError_t launch_group(const MarchParams& p, int num_sms, cudaStream_t s) {
+    MarchParams q = p;
+    q.tiles_x = (p.rx1 - p.rx0 + GroupTile<G>::W - 1) / GroupTile<G>::W;
+    q.tiles_y = (p.ry1 - p.ry0 + GroupTile<G>::H - 1) / GroupTile<G>::H;
+    return launch_persistent(march_group_kernel<DT, COMP, SHADE, BS, G, false>, q, (long long)q.tiles_x * q.tiles_y,
+                             num_sms, s);
+}
+
+// How a frame's rays are spread over lanes, by its 32-pixel tiles against the
+// warps the GPU holds (24 per SM). A frame ends when its longest ray does, and
+// on one lane such a ray takes as long as a thousand tiles: CT volume, 512^3
+// u16, shaded DVR, us by image and lanes per ray 1 / 2 / 4 / 8 / queue:
+//    160x90    (460 tiles)     229  174  117   84    96
+//    560x315   (5,530)         262  194  129  117   125
+//    800x450   (11,300)        237  181  157  162   141
+//    960x540   (16,200)        233  185  177  202   151
+//    1920x1080 (64,800)        314  353  427  682   256
+//    2560x1440 (115,200)       422  518  722 1179   371
+//    3840x2160 (259,200)       720 1014 1553 2584   710
+// (a 512x512x256 tube volume turns from 4 lanes to the queue between 11,300
+// and 16,200 tiles too). More lanes a ray cost more on runs through empty
+// space, which each lane of the group repeats, so they lose where the GPU is
+// full. The queue: one lane a ray, and the rays unfinished when the tiles run
+// out go on with 8 lanes each (half of a tube frame's gain with 4); it costs
+// the marching loop 3 % of its rate, which 4K frames do not get back.
+// MIP, MOP and MIDA go on to the end of the volume, so their rays are long
+// everywhere and the queue only adds to the work (512^3 MIP at 1080p 655 ->
+// 782 us, 1280x720 628 -> 970); they take 4 lanes up to 16,200 tiles (MIP 611
+// -> 394), 2 up to 28,800 (MIP 628 -> 595, MOP 534 -> 405), then one.
+// Pre-integration carries the previous sample along, a brick cache's use
+// marks depend on which samples are read, and first-hit rays end early: one
+// lane.
+template <int DT, int COMP, int SHADE, int BS, bool POOL>
+cudaError_t launch_t(const MarchParams& p, int num_sms, cudaStream_t s) {
+    const long long tiles = (long long)p.tiles_x * p.tiles_y;
+    constexpr bool ERT = COMP == VRC_DVR || COMP == VRC_ISO;
+    constexpr bool ALL = COMP == VRC_MIP || COMP == VRC_MOP || COMP == VRC_MIDA;
+    if constexpr (BS == 32 && !POOL && (ERT || ALL)) {
+        const long long warps = 24LL * num_sms;
+        if (2 * tiles <= 3 * warps) return launch_group<DT, COMP, SHADE, BS, 8>(p, num_sms, s);
+        if (tiles <= 3 * warps || (ALL && 2 * tiles <= 9 * warps))
+            return launch_group<DT, COMP, SHADE, BS, 4>(p, num_sms, s);
+        if constexpr (ALL) {
+            if (tiles <= 8 * warps) return launch_group<DT, COMP, SHADE, BS, 2>(p, num_sms, s);
+        } else if (p.queue && tiles <= 50 * warps) {
+            cudaError_t e = launch_persistent(march_kernel<DT, COMP, SHADE, BS, POOL, true>, p, tiles, num_sms, s);
+            if (e != cudaSuccess) return e;
+            return launch_persistent(march_group_kernel<DT, COMP, SHADE, BS, 8, true>, p, tiles, num_sms, s);
+        }
+    }
+    return launch_persistent(march_kernel<DT, COMP, SHADE, BS, POOL, false>, p, tiles, num_sms, s);
 }
 
 template <int DT, int COMP, int SHADE>

@@ -87,6 +87,12 @@ struct MarchParams {
     unsigned long long* counters;  // [samples, fetched, shaded]
     int* status;
     unsigned int* tile_counter;
+    // rays that march_kernel leaves to march_group_kernel: two float4 each
+    // (march_queue_bytes of them), their count and the second kernel's position;
+    // nullptr = every ray is marched to its end where it began
+    float4* queue;
+    unsigned* queue_count;
+    int* launches;               // host: counts the march kernels launched, nullptr = not counted
     int tiles_x, tiles_y;
     int tile_wshift;             // ray tile = (1 << tile_wshift) x (32 >> tile_wshift) pixels per warp
     int rx0, ry0, rx1, ry1;      // rendered pixel window [rx0, rx1) x [ry0, ry1) (the whole image by default)
@@ -113,6 +119,10 @@ struct MarchParams {
 #define VRC_OCC_DIST_CAP 16
 #endif
 constexpr int OCC_DIST_CAP = VRC_OCC_DIST_CAP;
+
+// Rays that can be under way at once: 8 CTAs of 256 threads (all that 64 warps
+// allow) on each SM.
+inline size_t march_queue_bytes(int num_sms) { return (size_t)num_sms * 2048 * 2 * sizeof(float4); }
 
 // Internal compositing code of the march kernels: DVR with pre-integrated
 // classification (no opacity correction, classify(previous, current)).
@@ -227,6 +237,7 @@ struct vrc_context {
     size_t dist_bytes = 0, dist_tmp_bytes = 0;
     int* d_prefix = nullptr;
     size_t prefix_bytes = 0;
+    void* d_queue = nullptr;  // unfinished rays between the march's two kernels (march_queue_bytes)
     unsigned long long* d_counters = nullptr;  // 4 counters + status + tile counter
     // what d_occ / d_occ_coarse hold: (volume uid, TF or table uid, table
     // width, domain lo/hi bits, skip cell edge); both are pure functions of it
