@@ -414,8 +414,8 @@ typedef struct {
     int kernels_per_launch;  /* kernel nodes in the captured graph */
 } vrc_batch_stats;
 
-/* Builds device descriptors and TF tables (allocating), orders requests
- * longest first and captures the launch sequence. Items are copied. */
+/* Builds device descriptors and TF tables (allocating), orders requests by
+ * voxel type and longest first within a type, and captures the launch sequence. Items are copied. */
 vrc_status vrc_batch_create(vrc_context* ctx, const vrc_batch_item* items, int n, vrc_batch** out);
 /* As vrc_batch_create, with each request isolated from the others: a request
  * that fails its checks (null or foreign handles, invalid parameters, a

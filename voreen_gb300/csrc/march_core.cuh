@@ -878,11 +878,13 @@ __device__ __forceinline__ float ray_setup(const MarchParams& P, float4 f, float
 
 // Colour of a sample's TF coordinate x: the entry's bytes / 255 (exact), alpha
 // from the per-byte table.
+template <bool GLOBAL_TF>
 __device__ __forceinline__ float4 tf_colour(const MarchParams& P, const uchar4* __restrict__ s_tf,
                                             const float* __restrict__ s_alpha, float rw) {
-    const uchar4 e8 = s_tf[(int)a_(m_(rw_to_tf(rw, P.tf_lo, P.tf_hi, P.tf_rcp), P.tf_wm1), 0.5f)];
+    const int i = (int)a_(m_(rw_to_tf(rw, P.tf_lo, P.tf_hi, P.tf_rcp), P.tf_wm1), 0.5f);
+    const uchar4 e8 = GLOBAL_TF ? __ldg(s_tf + i) : s_tf[i];
     const f2 rg = Vox<VRC_U8>::norm2(Vox<VRC_U8>::raw2(e8.x, e8.y));
-    return make_float4(lo2(rg), hi2(rg), Vox<VRC_U8>::norm(e8.z), s_alpha[e8.w]);
+    return make_float4(lo2(rg), hi2(rg), Vox<VRC_U8>::norm(e8.z), GLOBAL_TF ? __ldg(s_alpha + e8.w) : s_alpha[e8.w]);
 }
 
 // The empty-space test of one sample: whether its cell is empty for the ray
@@ -963,8 +965,8 @@ struct RayState {
 
 // One ray on one thread: the loop of cpuraycaster.cpp:239-317 with the GLSL
 // compositing. STOP: the ray is left unfinished (false) a sample or run after
-// *stop becomes set.
-template <int DT, int COMP, int SHADE, int BS, bool POOL, bool STOP>
+// *stop becomes set. GLOBAL_TF: the table is in global memory.
+template <int DT, int COMP, int SHADE, int BS, bool POOL, bool STOP, bool GLOBAL_TF = false>
 __device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __restrict__ s_tf,
                                           const float* __restrict__ s_alpha, float4 f, float4 l, int px, int py,
                                           const volatile int* stop, RayState& st, RayCounts& cnt) {
@@ -1104,7 +1106,7 @@ __device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __
                 c = __ldg(P.pi_table + (size_t)tf_index(cur, P.pi_res) * P.pi_res + tf_index(last, P.pi_res));
                 last = cur;
             } else {
-                c = tf_colour(P, s_tf, s_alpha, rw);
+                c = tf_colour<GLOBAL_TF>(P, s_tf, s_alpha, rw);
             }
             if (c.w > 0.f) {
                 float gmag2 = 0.f;
@@ -1221,7 +1223,7 @@ __device__ __forceinline__ void march_ray_group(const MarchParams& P, const ucha
                                             (p.ix - (bX << sh) + APRON_LO);
                 const Raw8 raw = load8<DT>(vox, S, BG::S2(P.L));
                 rw = a_(m_(tri8<DT>(raw, fx, fy, fz), P.rwm_scale), P.rwm_offset);
-                c = tf_colour(P, s_tf, s_alpha, rw);
+                c = tf_colour<false>(P, s_tf, s_alpha, rw);
                 if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) {
                     const F3 g = tl == 0.f ? clip_border_gradient(P, F3{p.sx, p.sy, p.sz}, F3{dx, dy, dz}, px, py)
                                            : central_gradient<DT, BS, false>(P, bricks, b, vox, raw, p, fx, fy, fz);
@@ -1423,12 +1425,13 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_group_kernel(
 }
 
 // Resident CTAs per SM of one kernel for a dynamic shared memory size,
-// queried once per (kernel, device, size): the attribute call and the
+// queried once per (kernel, device, size), and the kernel's shared memory limit
+// and carve-out set for `largest`, the most it is launched with: the attribute calls and the
 // occupancy query cost more host time than a frame's launch. Every march
 // instantiation has the same function type, so entries are keyed by the
 // kernel's address.
 template <typename K>
-cudaError_t resident_ctas(K k, size_t smem, int* per_sm) {
+cudaError_t resident_ctas(K k, size_t smem, size_t largest, int* per_sm) {
     struct Entry {
         const void* fn;
         int dev;
@@ -1447,10 +1450,6 @@ cudaError_t resident_ctas(K k, size_t smem, int* per_sm) {
             *per_sm = x.per_sm;
             return cudaSuccess;
         }
-    // the largest table (4096 entries) once per device; smaller ones fit under
-    // it (a kernel that stages no table, pre-integration, asks for the 256 alphas)
-    const size_t head = 256 * sizeof(float);
-    const size_t largest = smem > head ? head + (size_t)4096 * sizeof(uchar4) : head;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)largest);
     if (e != cudaSuccess) return e;
     int n = 0, reserved = 0, per_sm_bytes = 0;
@@ -1480,7 +1479,10 @@ inline size_t tf_smem(const MarchParams& p) { return 256 * sizeof(float) + (size
 template <typename K>
 cudaError_t launch_persistent(K k, const MarchParams& p, long long tiles, int num_sms, cudaStream_t s) {
     int per_sm = 0;
-    cudaError_t e = resident_ctas(k, tf_smem(p), &per_sm);
+    // the largest table (4096 entries) once per device; smaller ones fit under
+    // it (a kernel that stages no table, pre-integration, has the 256 alphas)
+    const size_t largest = 256 * sizeof(float) + (p.tf_width > 0 ? (size_t)4096 * sizeof(uchar4) : 0);
+    cudaError_t e = resident_ctas(k, tf_smem(p), largest, &per_sm);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     long long grid = (long long)num_sms * per_sm;

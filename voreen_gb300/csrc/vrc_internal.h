@@ -177,10 +177,12 @@ cudaError_t launch_preint_exact(const float4* tb, const uint8_t* a8, const float
 cudaError_t launch_entry_exit(const MarchParams& p, float4* entry, float4* exitp, cudaStream_t s);
 // Batch: zero the per-launch state and stamp the start time, then one
 // persistent launch over every request's ray tiles (tile_prefix[r] = first
-// tile of request r in launch order; n + 1 entries).
+// tile of request r in launch order; n + 1 entries). bricks32: all their
+// volumes have 32^3 bricks.
 cudaError_t launch_batch_begin(unsigned long long* state, int nreq, cudaStream_t s);
 cudaError_t launch_march_batch(const BatchReq* reqs, int nreq, const unsigned* tile_prefix, unsigned total_tiles,
-                               unsigned long long* state, int compositing, int shading, int num_sms, cudaStream_t s);
+                               unsigned long long* state, int compositing, int shading, bool bricks32, int num_sms,
+                               cudaStream_t s);
 // Copies brick ids[i] of `pool` to slot dst[i] of `cache` (brick_stride_bytes
 // each), i in [0, n).
 cudaError_t launch_brick_gather(const void* pool, const long long* ids, const long long* dst, long long n,
