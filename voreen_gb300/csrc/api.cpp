@@ -335,8 +335,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: copy: ") + cudaGetErrorString(e));
         lin = staging;
     }
-    if ((e = vrc::launch_brick_build(lin, desc->dtype, L, v->d_bricks, ctx->stream)) != cudaSuccess ||
-        (e = vrc::launch_brick_minmax(v->d_bricks, desc->dtype, L, v->d_bmin, v->d_bmax, ctx->stream)) != cudaSuccess)
+    if ((e = vrc::launch_brick_build(lin, desc->dtype, L, v->d_bricks, ctx->stream)) != cudaSuccess)
         return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: kernel: ") + cudaGetErrorString(e));
     // finer empty-space cells (2^3, 4^3, 8^3, 16^3) below the brick size;
     // 2^3 cells (8 bytes of tables per 8 voxels) only up to
@@ -355,9 +354,22 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             (e = cudaMalloc((void**)&lv.d_max, lv.count() * sizeof(float))) != cudaSuccess)
             return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: cell table allocation failed");
         v->bytes += 2 * lv.count() * sizeof(float);
-        if ((e = vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, C, lv.d_min, lv.d_max, ctx->stream)) != cudaSuccess)
+        // the finest level from the voxels, the others each from the one below
+        const vrc_cell_level* fine = li > 0 && v->levels[li - 1].d_max ? &v->levels[li - 1] : nullptr;
+        e = fine ? vrc::launch_coarser_minmax(fine->d_min, fine->d_max, fine->nc, 2, lv.nc, lv.d_min, lv.d_max, ctx->stream)
+                 : vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, C, lv.d_min, lv.d_max, ctx->stream);
+        if (e != cudaSuccess)
             return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: cell kernel: ") + cudaGetErrorString(e));
     }
+    // the bricks' from the coarsest cells (half a brick, or a quarter of a 64^3 one)
+    const vrc_cell_level* half = nullptr;
+    for (const auto& lv : v->levels)
+        if (lv.d_max && (lv.C * 2 == L.B || (lv.C * 4 == L.B && L.B == 64))) half = &lv;
+    e = half ? vrc::launch_coarser_minmax(half->d_min, half->d_max, half->nc, L.B / half->C, L.nb, v->d_bmin, v->d_bmax,
+                                          ctx->stream)
+             : vrc::launch_brick_minmax(v->d_bricks, desc->dtype, L, v->d_bmin, v->d_bmax, ctx->stream);
+    if (e != cudaSuccess)
+        return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: brick kernel: ") + cudaGetErrorString(e));
     std::vector<float> mn(L.nbricks()), mx(L.nbricks());
     if ((e = cudaMemcpyAsync(mn.data(), v->d_bmin, mn.size() * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream)) !=
             cudaSuccess ||

@@ -199,6 +199,9 @@ cudaError_t launch_brick_minmax(const void* bricks, int dtype, const BrickLayout
 // plus one voxel on the high side (clamped), from the linear volume.
 cudaError_t launch_cell_minmax(const void* linear, int dtype, const int dims[3], int C, float* cmin, float* cmax,
                                cudaStream_t s);
+// The same for cells of `factor` (2 or 4) times the edge, from a level's own.
+cudaError_t launch_coarser_minmax(const float* fmin, const float* fmax, const int fnc[3], int factor, const int nc[3],
+                                  float* cmin, float* cmax, cudaStream_t s);
 // Writes ceil(ncells / 32) words: bit (c & 31) of word (c >> 5) is set when
 // cell c may hold a sample with TF alpha > 0.
 cudaError_t launch_occupancy(const float* bmin, const float* bmax, long long ncells, const int* alpha_prefix,
