@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "../../include/vrc_nn.h"
 
 namespace {
@@ -42,6 +44,19 @@ __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uin
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// 16 bytes global -> shared in the background; not valid: zeros.
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+    const int n = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async16_l1(uint32_t dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int LEFT> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(LEFT) : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // Forward 3x3 convolution (stride 1, zero padding 1).
 // CTA: an output tile of TH rows x 16 columns, all COUT channels; 8 warps,
@@ -49,84 +64,134 @@ __device__ __forceinline__ void mma_bf16(float* d, uint32_t a0, uint32_t a1, uin
 // Per 16-channel input chunk the CTA stages the (TH+2) x 18 input halo and the
 // 9 x COUT x 16 weights in shared memory (rows padded to 24 BF16 so ldmatrix
 // rows fall on distinct banks), then runs 9 taps x COUT/8 MMAs per m-tile.
+//
+// The bound is the mma.sync rate; what kept the kernel from it were the loads
+// of a chunk, waited for between two barriers, and ldmatrix: a row's operand
+// was read again for each tap row that uses it. Two sets of stages let the
+// next chunk's copies (cp.async, zero-filled outside the image) run under this
+// chunk's MMAs. Each accumulator adds its products in the order of chunks and taps, as
+// before, so the results keep their bits. 960x540 96 -> 32 103 -> 93 us
+// (310 TFLOP/s), 480x270 192 -> 64 105 -> 90, 960x540 32 -> 16 28 -> 23.
 constexpr int PIX_PAD = 24;  // bf16 per staged pixel / weight row (16 used)
+
+template <int COUT, int RPW> struct FwdTile {
+    static constexpr int TH = 8 * RPW;
+    static constexpr int IN = (TH + 2) * 18 * PIX_PAD;      // bf16 of one staged input halo
+    static constexpr int STAGE = IN + 9 * COUT * PIX_PAD;  // ... and of a stage
+    // up to 32 output channels a row's operands stay in registers for the next
+    // tap row, and the weights, the same for every CTA, are copied through L1
+    // (960x540 16 -> 32: 37 us past it, 25 through it); with 64 the registers
+    // spill and the weights push the input out of L1 (480x270 64 -> 64: 38.9 us
+    // so, 35.7 otherwise)
+    static constexpr bool KEEP = COUT <= 32;
+    static constexpr int PIECES = ((TH + 2) * 36 + 255) / 256;  // 16-byte pieces of the halo a thread copies
+    static constexpr size_t BYTES = STAGE * sizeof(__nv_bfloat16);
+};
 
 // Optional fused input [up2(A) | B]: channels [0, Ca) come from A at half
 // resolution (nearest 2x upsample on load) and [Ca, Ca + Cb) from B; Cin =
 // Ca + Cb and `in` is A. With in_b == nullptr the input is `in` as is.
 template <int COUT, int RPW>
-__global__ void __launch_bounds__(256) conv3x3_fwd_kernel(const __nv_bfloat16* __restrict__ in, int N, int H, int W,
-                                                          int Cin, const __nv_bfloat16* __restrict__ wt,
-                                                          const float* __restrict__ bias, int relu, void* out,
-                                                          int out_f32, const __nv_bfloat16* __restrict__ in_b,
-                                                          int Ca) {
-    constexpr int TH = 8 * RPW;
+__global__ void __launch_bounds__(256, COUT <= 32 ? 3 : (COUT == 64 ? 2 : 1))
+    conv3x3_fwd_kernel(const __nv_bfloat16* __restrict__ in, int N, int H, int W, int Cin,
+                       const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias, int relu, void* out,
+                       int out_f32, const __nv_bfloat16* __restrict__ in_b, int Ca) {
+    using FT = FwdTile<COUT, RPW>;
     constexpr int NT = COUT / 8;
-    extern __shared__ __align__(16) __nv_bfloat16 smem[];
-    __nv_bfloat16* s_in = smem;                                   // [TH+2][18][PIX_PAD]
-    __nv_bfloat16* s_w = smem + (TH + 2) * 18 * PIX_PAD;          // [9][COUT][PIX_PAD]
+    extern __shared__ __align__(16) __nv_bfloat16 smem[];  // [2] x { [TH+2][18][PIX_PAD], [9][COUT][PIX_PAD] }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int x0 = blockIdx.x * 16, y0 = blockIdx.y * TH, n = blockIdx.z;
+    const int x0 = blockIdx.x * 16, y0 = blockIdx.y * FT::TH, n = blockIdx.z;
     float acc[RPW][NT][4];
 #pragma unroll
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
         for (int j = 0; j < NT; ++j) acc[r][j][0] = acc[r][j][1] = acc[r][j][2] = acc[r][j][3] = 0.f;
 
-    for (int c0 = 0; c0 < Cin; c0 += 16) {
-        // stage the input halo: (TH+2) x 18 pixels x 16 channels, 2 x 16 B per pixel
-        for (int i = tid; i < (TH + 2) * 18 * 2; i += 256) {
-            const int half = i & 1, pix = i >> 1;
-            const int ry = pix / 18, rx = pix % 18;
-            const int gy = y0 + ry - 1, gx = x0 + rx - 1;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gy >= 0 && gy < H && gx >= 0 && gx < W) {
-                if (in_b == nullptr) {
-                    v = *reinterpret_cast<const uint4*>(in + (((size_t)n * H + gy) * W + gx) * Cin + c0 + half * 8);
-                } else if (c0 < Ca) {
-                    const int Hh = H >> 1, Wh = W >> 1;
-                    v = *reinterpret_cast<const uint4*>(in + (((size_t)n * Hh + (gy >> 1)) * Wh + (gx >> 1)) * Ca + c0 +
-                                                        half * 8);
-                } else {
-                    const int Cb = Cin - Ca;
-                    v = *reinterpret_cast<const uint4*>(in_b + (((size_t)n * H + gy) * W + gx) * Cb + (c0 - Ca) +
-                                                        half * 8);
-                }
-            }
-            *reinterpret_cast<uint4*>(s_in + (ry * 18 + rx) * PIX_PAD + half * 8) = v;
+    // this thread's pieces of the halo: (TH+2) x 18 pixels x 16 channels, 2 x 16 B per pixel
+    const int Cb = Cin - Ca;
+    size_t from[FT::PIECES], from_b[FT::PIECES];  // element of the piece in `in` and in_b, chunk 0
+    bool valid[FT::PIECES];
+#pragma unroll
+    for (int k = 0; k < FT::PIECES; ++k) {
+        const int i = tid + 256 * k, half = i & 1, pix = i >> 1;
+        const int gy = y0 + pix / 18 - 1, gx = x0 + pix % 18 - 1;
+        valid[k] = gy >= 0 && gy < H && gx >= 0 && gx < W;
+        from[k] = from_b[k] = 0;
+        if (!valid[k]) continue;
+        if (in_b == nullptr) {
+            from[k] = (((size_t)n * H + gy) * W + gx) * Cin + half * 8;
+        } else {
+            from[k] = (((size_t)n * (H >> 1) + (gy >> 1)) * (W >> 1) + (gx >> 1)) * Ca + half * 8;
+            from_b[k] = (((size_t)n * H + gy) * W + gx) * Cb + half * 8;
         }
-        // stage weights [tap][cout][16]
+    }
+    const uint32_t s0 = smem_u32(smem);
+    auto stage = [&](int c0, int set) {
+        const uint32_t si = s0 + set * FT::STAGE * 2, sw = si + FT::IN * 2;
+#pragma unroll
+        for (int k = 0; k < FT::PIECES; ++k) {
+            const int i = tid + 256 * k;
+            if (i < (FT::TH + 2) * 36) {
+                const __nv_bfloat16* p = in_b == nullptr || c0 < Ca ? in + from[k] + c0 : in_b + from_b[k] + (c0 - Ca);
+                cp_async16(si + ((i >> 1) * PIX_PAD + (i & 1) * 8) * 2, valid[k] ? p : in, valid[k]);
+            }
+        }
         for (int i = tid; i < 9 * COUT * 2; i += 256) {
             const int half = i & 1, row = i >> 1;  // row = tap * COUT + co
             const int tap = row / COUT, co = row % COUT;
-            const uint4 v = *reinterpret_cast<const uint4*>(wt + ((size_t)co * 9 + tap) * Cin + c0 + half * 8);
-            *reinterpret_cast<uint4*>(s_w + row * PIX_PAD + half * 8) = v;
+            const __nv_bfloat16* p = wt + ((size_t)co * 9 + tap) * Cin + c0 + half * 8;
+            const uint32_t to = sw + (row * PIX_PAD + half * 8) * 2;
+            if (FT::KEEP) cp_async16_l1(to, p);
+            else cp_async16(to, p, true);
+        }
+        cp_async_commit();
+    };
+    stage(0, 0);
+    for (int c0 = 0, set = 0; c0 < Cin; c0 += 16, set ^= 1) {
+        if (c0 + 16 < Cin) {
+            stage(c0 + 16, set ^ 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
         }
         __syncthreads();
+        const uint32_t sa = s0 + set * FT::STAGE * 2 + ((warp * RPW * 18 + (lane & 15)) * PIX_PAD + (lane >> 4) * 8) * 2;
+        // two n-tiles a load: lanes 0-15 -> tile j (k 0 / 8), lanes 16-31 -> tile j + 1
+        const uint32_t sb = s0 + (set * FT::STAGE + FT::IN) * 2 +
+                            (((lane >> 4) * 8 + (lane & 7)) * PIX_PAD + ((lane >> 3) & 1) * 8) * 2;
+        uint32_t a[RPW][3][4];
+        auto load_row = [&](int r, int row) {
 #pragma unroll
-        for (int tap = 0; tap < 9; ++tap) {
-            const int kh = tap / 3, kw = tap % 3;
-            uint32_t a[RPW][4];
+            for (int kw = 0; kw < 3; ++kw)
+                ldsm_x4(sa + (row * 18 + kw) * PIX_PAD * 2, a[r][kw][0], a[r][kw][1], a[r][kw][2], a[r][kw][3]);
+        };
+#pragma unroll
+        for (int kh = 0; kh < 3; ++kh) {
+            // the rows move up by one and the last is new, or all are read again
 #pragma unroll
             for (int r = 0; r < RPW; ++r) {
-                const int row = warp * RPW + r + kh;
-                const __nv_bfloat16* p = s_in + (row * 18 + kw + (lane & 15)) * PIX_PAD + (lane >> 4) * 8;
-                ldsm_x4(smem_u32(p), a[r][0], a[r][1], a[r][2], a[r][3]);
-            }
+                if (FT::KEEP && kh > 0 && r + 1 < RPW) {
 #pragma unroll
-            for (int j = 0; j < NT; j += 2) {
-                // two n-tiles: lanes 0-15 -> tile j (k 0 / 8), lanes 16-31 -> tile j + 1
-                const int jj = j + (lane >> 4);
-                const int co = (jj < NT ? jj : j) * 8 + (lane & 7);
-                const __nv_bfloat16* p = s_w + (tap * COUT + co) * PIX_PAD + ((lane >> 3) & 1) * 8;
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4(smem_u32(p), b0, b1, b2, b3);
+                    for (int kw = 0; kw < 3; ++kw)
 #pragma unroll
-                for (int r = 0; r < RPW; ++r) {
-                    mma_bf16(acc[r][j], a[r][0], a[r][1], a[r][2], a[r][3], b0, b1);
-                    if (j + 1 < NT) mma_bf16(acc[r][j + 1], a[r][0], a[r][1], a[r][2], a[r][3], b2, b3);
+                        for (int q = 0; q < 4; ++q) a[r][kw][q] = a[r + 1][kw][q];
+                } else {
+                    load_row(r, r + kh);
                 }
             }
+#pragma unroll
+            for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+                for (int j = 0; j < NT; j += 2) {
+                    uint32_t b0, b1, b2, b3;
+                    ldsm_x4(sb + ((kh * 3 + kw) * COUT + j * 8) * PIX_PAD * 2, b0, b1, b2, b3);
+#pragma unroll
+                    for (int r = 0; r < RPW; ++r) {
+                        const uint32_t* q = a[r][kw];
+                        mma_bf16(acc[r][j], q[0], q[1], q[2], q[3], b0, b1);
+                        mma_bf16(acc[r][j + 1], q[0], q[1], q[2], q[3], b2, b3);
+                    }
+                }
         }
         __syncthreads();
     }
@@ -168,121 +233,156 @@ template <int COUT, int RPW>
 cudaError_t conv_fwd_t(const __nv_bfloat16* in, int N, int H, int W, int Cin, const __nv_bfloat16* w,
                        const float* bias, int relu, void* out, int out_f32, cudaStream_t s,
                        const __nv_bfloat16* in_b = nullptr, int Ca = 0) {
-    constexpr int TH = 8 * RPW;
-    const size_t smem = ((TH + 2) * 18 * PIX_PAD + 9 * COUT * PIX_PAD) * sizeof(__nv_bfloat16);
+    using FT = FwdTile<COUT, RPW>;
     auto k = conv3x3_fwd_kernel<COUT, RPW>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * FT::BYTES));
     if (e != cudaSuccess) return e;
-    dim3 grid((W + 15) / 16, (H + TH - 1) / TH, N);
-    k<<<grid, 256, smem, s>>>(in, N, H, W, Cin, w, bias, relu, out, out_f32, in_b, Ca);
+    dim3 grid((W + 15) / 16, (H + FT::TH - 1) / FT::TH, N);
+    // one chunk needs one set of stages
+    k<<<grid, 256, (Cin > 16 ? 2 : 1) * FT::BYTES, s>>>(in, N, H, W, Cin, w, bias, relu, out, out_f32, in_b, Ca);
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // Weight gradient: dW[co][tap][ci] += sum_p dout[p][co] * in[p + tap - 1][ci]
 // (and dbias[co] += sum_p dout[p][co] when requested).
-// CTA: one tap, all COUT output channels, a 64-channel input block, and a
-// run of PIX_TILES 8x16 pixel tiles; per tile it stages dout (128 x COUT) and
-// the shifted input (128 x 64), rows padded to stride+8 BF16, and runs
-// 8 k-steps of 16 pixels: A = dout^T via ldmatrix.trans, B = input via
-// ldmatrix.trans. Partial sums are added to the FP32 gradients atomically.
+// CTA: the three taps of one tap row, all COUT output channels, a 64-channel
+// input block, and a run of 8x16 pixel tiles; per tile it stages dout (128 x
+// COUT) and the rows of the input it meets (8 x 18 pixels x 64), rows padded
+// to stride+8 BF16, and runs 8 k-steps of 16 pixels a tap: A = dout^T via
+// ldmatrix.trans, B = input via ldmatrix.trans, the taps one pixel apart.
+// Partial sums are added to the FP32 gradients atomically, two at a time.
+//
+// One CTA a tap (9 loads of the same pixels) and runs of 32 tiles left 162
+// CTAs for 152 SMs at 8 x 96 x 96, each waiting for one tile's loads at a time:
+// 41 TFLOP/s. Now dout and input are read 3 times, the next tile's copies run
+// under this one's MMAs, and the runs are as short as two CTAs per SM ask.
+// 64 -> 64, 8 x 96 x 96: 99 -> 29 us.
 constexpr int WG_CI = 64;
+constexpr int WGRAD_CTAS = 304;
+
+template <int COUT> struct WgradTile {
+    static constexpr int DS = COUT + 8, IS = WG_CI + 8;  // padded row strides (bf16)
+    static constexpr int D = 128 * DS, STAGE = D + 8 * 18 * IS;
+    static constexpr size_t BYTES = 2 * STAGE * sizeof(__nv_bfloat16);
+};
 
 template <int COUT>
-__global__ void __launch_bounds__(256) conv3x3_wgrad_kernel(const __nv_bfloat16* __restrict__ in,
-                                                            const __nv_bfloat16* __restrict__ dout, int N, int H,
-                                                            int W, int Cin, float* dw, float* dbias,
-                                                            int tiles_per_cta) {
+__global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
+    conv3x3_wgrad_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout, int N, int H,
+                         int W, int Cin, float* dw, float* dbias, int tiles_per_cta) {
+    using WT = WgradTile<COUT>;
     constexpr int MT = COUT / 16;               // m16 tiles along COUT
     constexpr int NG = 8 / MT;                  // warps sharing one m tile, each owns 8/NG n-tiles
     constexpr int NTW = (WG_CI / 8) / NG;       // n8 tiles per warp
-    constexpr int DS = COUT + 8, IS = WG_CI + 8;  // padded row strides (bf16)
-    extern __shared__ __align__(16) __nv_bfloat16 smem[];
-    __nv_bfloat16* s_d = smem;                  // [128][DS]
-    __nv_bfloat16* s_i = smem + 128 * DS;       // [128][IS]
+    extern __shared__ __align__(16) __nv_bfloat16 smem[];  // [2] x { dout [128][DS], input [8][18][IS] }
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tap = blockIdx.y, kh = tap / 3, kw = tap % 3;
-    const int ci0 = blockIdx.z * WG_CI;
+    const int kh = blockIdx.y, ci0 = blockIdx.z * WG_CI;
     const int mt = warp % MT, ng = warp / MT;
     const int tiles_x = (W + 15) / 16, tiles_y = (H + 7) / 8, ntiles = tiles_x * tiles_y * N;
-    float acc[NTW][4];
+    float acc[3][NTW][4];
 #pragma unroll
-    for (int j = 0; j < NTW; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) acc[t][j][0] = acc[t][j][1] = acc[t][j][2] = acc[t][j][3] = 0.f;
+    // dbias: channel tid % COUT, the tile's pixels shared by 256 / COUT threads
+    constexpr int PARTS = 256 / COUT;
+    const bool sums_bias = dbias && kh == 0 && blockIdx.z == 0;
     float bsum = 0.f;
-    const int t_begin = blockIdx.x * tiles_per_cta, t_end = min(ntiles, t_begin + tiles_per_cta);
-    for (int tile = t_begin; tile < t_end; ++tile) {
+    const uint32_t s0 = smem_u32(smem);
+    auto stage = [&](int tile, int set) {
         const int n = tile / (tiles_x * tiles_y), rem = tile % (tiles_x * tiles_y);
         const int y0 = (rem / tiles_x) * 8, x0 = (rem % tiles_x) * 16;
-        // stage dout rows (128 pixels x COUT) and shifted input (128 x 64)
+        const uint32_t sd = s0 + set * WT::STAGE * 2, si = sd + WT::D * 2;
         for (int i = tid; i < 128 * (COUT / 8); i += 256) {
             const int p = i / (COUT / 8), v8 = i % (COUT / 8);
             const int y = y0 + p / 16, x = x0 + p % 16;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (y < H && x < W) v = *reinterpret_cast<const uint4*>(dout + (((size_t)n * H + y) * W + x) * COUT + v8 * 8);
-            *reinterpret_cast<uint4*>(s_d + p * DS + v8 * 8) = v;
+            const bool ok = y < H && x < W;
+            cp_async16(sd + (p * WT::DS + v8 * 8) * 2, ok ? dout + (((size_t)n * H + y) * W + x) * COUT + v8 * 8 : dout, ok);
         }
-        for (int i = tid; i < 128 * (WG_CI / 8); i += 256) {
+        for (int i = tid; i < 8 * 18 * (WG_CI / 8); i += 256) {
             const int p = i / (WG_CI / 8), v8 = i % (WG_CI / 8);
-            const int y = y0 + p / 16, x = x0 + p % 16;
-            const int gy = y + kh - 1, gx = x + kw - 1;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (y < H && x < W && gy >= 0 && gy < H && gx >= 0 && gx < W && ci0 + v8 * 8 < Cin)
-                v = *reinterpret_cast<const uint4*>(in + (((size_t)n * H + gy) * W + gx) * Cin + ci0 + v8 * 8);
-            *reinterpret_cast<uint4*>(s_i + p * IS + v8 * 8) = v;
+            const int gy = y0 + p / 18 + kh - 1, gx = x0 + p % 18 - 1;
+            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W && ci0 + v8 * 8 < Cin;
+            cp_async16(si + (p * WT::IS + v8 * 8) * 2, ok ? in + (((size_t)n * H + gy) * W + gx) * Cin + ci0 + v8 * 8 : in, ok);
+        }
+        cp_async_commit();
+    };
+    const int t_begin = blockIdx.x * tiles_per_cta, t_end = min(ntiles, t_begin + tiles_per_cta);
+    if (t_begin < t_end) stage(t_begin, 0);
+    for (int tile = t_begin, set = 0; tile < t_end; ++tile, set ^= 1) {
+        if (tile + 1 < t_end) {
+            stage(tile + 1, set ^ 1);
+            cp_async_wait<1>();
+        } else {
+            cp_async_wait<0>();
         }
         __syncthreads();
-        if (dbias && tap == 0 && blockIdx.z == 0)
-            for (int co = tid; co < COUT; co += 256)
-                for (int p = 0; p < 128; ++p) bsum += __bfloat162float(s_d[p * DS + co]);
+        const __nv_bfloat16 *s_d = smem + set * WT::STAGE, *s_i = s_d + WT::D;
+        if (sums_bias)
+            for (int p = tid / COUT; p < 128; p += PARTS) bsum += __bfloat162float(s_d[p * WT::DS + tid % COUT]);
 #pragma unroll
-        for (int k0 = 0; k0 < 128; k0 += 16) {
+        for (int row = 0; row < 8; ++row) {
             // A (m = co, k = pixel): stored [pixel][co] -> ldmatrix.trans
             uint32_t a0, a1, a2, a3;
             {
-                const int p = k0 + ((lane >> 4) << 3) + (lane & 7);
+                const int p = row * 16 + ((lane >> 4) << 3) + (lane & 7);
                 const int co = mt * 16 + ((lane >> 3) & 1) * 8;
-                ldsm_x4_t(smem_u32(s_d + p * DS + co), a0, a1, a2, a3);
+                ldsm_x4_t(smem_u32(s_d + p * WT::DS + co), a0, a1, a2, a3);
             }
 #pragma unroll
-            for (int j = 0; j < NTW; j += 2) {
-                // B (k = pixel, n = ci): stored [pixel][ci] -> ldmatrix.trans; two n-tiles
-                const int nt = ng * NTW + j + (lane >> 4);
-                const int p = k0 + ((lane >> 3) & 1) * 8 + (lane & 7);
-                uint32_t b0, b1, b2, b3;
-                ldsm_x4_t(smem_u32(s_i + p * IS + nt * 8), b0, b1, b2, b3);
-                mma_bf16(acc[j], a0, a1, a2, a3, b0, b1);
-                if (j + 1 < NTW) mma_bf16(acc[j + 1], a0, a1, a2, a3, b2, b3);
-            }
+            for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+                for (int j = 0; j < NTW; j += 2) {
+                    // B (k = pixel, n = ci): stored [pixel][ci] -> ldmatrix.trans; two n-tiles
+                    const int nt = ng * NTW + j + (lane >> 4);
+                    const int p = row * 18 + kw + ((lane >> 3) & 1) * 8 + (lane & 7);
+                    uint32_t b0, b1, b2, b3;
+                    ldsm_x4_t(smem_u32(s_i + p * WT::IS + nt * 8), b0, b1, b2, b3);
+                    mma_bf16(acc[kw][j], a0, a1, a2, a3, b0, b1);
+                    if (j + 1 < NTW) mma_bf16(acc[kw][j + 1], a0, a1, a2, a3, b2, b3);
+                }
         }
         __syncthreads();
     }
     const int g = lane >> 2, t = lane & 3;
+    const bool pairs = reinterpret_cast<uintptr_t>(dw) % 8 == 0;  // Cin and ci are even
 #pragma unroll
-    for (int j = 0; j < NTW; ++j) {
-        const int ci = ci0 + (ng * NTW + j) * 8 + 2 * t;
-        const int co = mt * 16 + g;
-        if (ci < Cin) {
-            atomicAdd(dw + ((size_t)co * 9 + tap) * Cin + ci, acc[j][0]);
-            atomicAdd(dw + ((size_t)co * 9 + tap) * Cin + ci + 1, acc[j][1]);
-            atomicAdd(dw + ((size_t)(co + 8) * 9 + tap) * Cin + ci, acc[j][2]);
-            atomicAdd(dw + ((size_t)(co + 8) * 9 + tap) * Cin + ci + 1, acc[j][3]);
+    for (int kw = 0; kw < 3; ++kw)
+#pragma unroll
+        for (int j = 0; j < NTW; ++j) {
+            const int ci = ci0 + (ng * NTW + j) * 8 + 2 * t;
+            const int co = mt * 16 + g, tap = kh * 3 + kw;
+            if (ci >= Cin) continue;
+            float* d0 = dw + ((size_t)co * 9 + tap) * Cin + ci;
+            float* d1 = d0 + (size_t)8 * 9 * Cin;
+            if (pairs) {
+                atomicAdd(reinterpret_cast<float2*>(d0), make_float2(acc[kw][j][0], acc[kw][j][1]));
+                atomicAdd(reinterpret_cast<float2*>(d1), make_float2(acc[kw][j][2], acc[kw][j][3]));
+            } else {
+                atomicAdd(d0, acc[kw][j][0]);
+                atomicAdd(d0 + 1, acc[kw][j][1]);
+                atomicAdd(d1, acc[kw][j][2]);
+                atomicAdd(d1 + 1, acc[kw][j][3]);
+            }
         }
-    }
-    if (dbias && tap == 0 && blockIdx.z == 0)
-        for (int co = tid; co < COUT; co += 256) atomicAdd(dbias + co, bsum);
+    if (sums_bias) atomicAdd(dbias + tid % COUT, bsum);
 }
 
 template <int COUT>
 cudaError_t conv_wgrad_t(const __nv_bfloat16* in, const __nv_bfloat16* dout, int N, int H, int W, int Cin, float* dw,
                          float* dbias, cudaStream_t s) {
-    const size_t smem = (128 * (COUT + 8) + 128 * (WG_CI + 8)) * sizeof(__nv_bfloat16);
+    using WT = WgradTile<COUT>;
     auto k = conv3x3_wgrad_kernel<COUT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WT::BYTES);
     if (e != cudaSuccess) return e;
     const int ntiles = ((W + 15) / 16) * ((H + 7) / 8) * N;
-    const int per = 32;
-    dim3 grid((ntiles + per - 1) / per, 9, (Cin + WG_CI - 1) / WG_CI);
-    k<<<grid, 256, smem, s>>>(in, dout, N, H, W, Cin, dw, dbias, per);
+    const int blocks = 3 * ((Cin + WG_CI - 1) / WG_CI);
+    // two CTAs an SM in all; at most 32 tiles a CTA, as sums of more rounded differently
+    const int runs = (WGRAD_CTAS + blocks - 1) / blocks;
+    const int per = max(1, min(32, (ntiles + runs - 1) / runs));
+    dim3 grid((ntiles + per - 1) / per, 3, (Cin + WG_CI - 1) / WG_CI);
+    k<<<grid, 256, WT::BYTES, s>>>(in, dout, N, H, W, Cin, dw, dbias, per);
     return cudaGetLastError();
 }
 
@@ -296,18 +396,35 @@ __global__ void relu_bwd_kernel(const __nv_bfloat16* y, __nv_bfloat16* dy, long 
 }
 
 // 2x2 average pool times `scale`, NHWC (H, W even); scale 4 gives the
-// sum-pooling that is the backward of the nearest 2x upsample
-__global__ void avgpool_kernel(const __nv_bfloat16* in, int N, int H, int W, int C, float scale, __nv_bfloat16* out) {
-    const int Ho = H / 2, Wo = W / 2;
-    const long long n = (long long)N * Ho * Wo * C;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int c = (int)(i % C);
-        long long r = i / C;
-        const int x = (int)(r % Wo), y = (int)((r / Wo) % Ho), b = (int)(r / ((long long)Wo * Ho));
-        const __nv_bfloat16* p = in + (((size_t)b * H + 2 * y) * W + 2 * x) * C + c;
-        const float s = __bfloat162float(p[0]) + __bfloat162float(p[C]) + __bfloat162float(p[(size_t)W * C]) +
-                        __bfloat162float(p[(size_t)W * C + C]);
-        out[i] = __float2bfloat16(0.25f * scale * s);
+// sum-pooling that is the backward of the nearest 2x upsample. HBM is the
+// bound. Eight channels a thread where C and the pointers allow 16-byte
+// accesses, else one; a channel a thread took five 64-bit divisions for 10
+// bytes (960x540x32: 27 -> 8.4 us).
+__device__ __forceinline__ float pool4(__nv_bfloat16 a, __nv_bfloat16 b, __nv_bfloat16 c, __nv_bfloat16 d, float scale) {
+    const float s = __bfloat162float(a) + __bfloat162float(b) + __bfloat162float(c) + __bfloat162float(d);
+    return 0.25f * scale * s;
+}
+template <int V>
+__global__ void avgpool_kernel(const __nv_bfloat16* __restrict__ in, int rows, int H, int W, int C, float scale,
+                               __nv_bfloat16* __restrict__ out) {
+    struct alignas(2 * V) Vec {
+        __nv_bfloat16 v[V];
+    };
+    const int Ho = H / 2, Wo = W / 2, CV = C / V;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
+        const int b = row / Ho, y = row - b * Ho;
+        const Vec* p = reinterpret_cast<const Vec*>(in + ((size_t)b * H + 2 * y) * W * C);
+        const Vec* q = p + (size_t)W * CV;
+        Vec* o = reinterpret_cast<Vec*>(out + (size_t)row * Wo * C);
+        for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)Wo * CV;
+             i += (long long)gridDim.x * blockDim.x) {
+            const long long x = i / CV, at = 2 * x * CV + (i - x * CV);
+            const Vec p0 = p[at], p1 = p[at + CV], q0 = q[at], q1 = q[at + CV];
+            Vec r;
+#pragma unroll
+            for (int k = 0; k < V; ++k) r.v[k] = __float2bfloat16(pool4(p0.v[k], p1.v[k], q0.v[k], q1.v[k], scale));
+            o[i] = r;
+        }
     }
 }
 // backward of avgpool: din = dout / 4 replicated; with `scale` = 1 it is the
@@ -358,7 +475,37 @@ __device__ __forceinline__ float bilerp_base(const float* base, int b, int H, in
     const float v10 = p[((size_t)y1 * W + x0) * 4 + k], v11 = p[((size_t)y1 * W + x1) * 4 + k];
     return (v00 * (1.f - fx) + v01 * fx) * (1.f - fy) + (v10 * (1.f - fx) + v11 * fx) * fy;
 }
-__global__ void head_fwd_kernel(const float* feat16, const float* base, int N, int H, int W, float* out) {
+// An output pixel a thread: its four features and four base pixels are one
+// 16-byte load each. HBM is the bound (64 + 16 bytes a low-resolution pixel
+// read, 64 written). A channel a thread, with 64-bit divisions and scalar
+// loads, took 57.7 us at 960x540, this 16.6.
+__device__ __forceinline__ float4 bilerp_base4(const float4* __restrict__ p, int H, int W, int oy, int ox) {
+    const float sy = fmaxf((oy + 0.5f) * 0.5f - 0.5f, 0.f), sx = fmaxf((ox + 0.5f) * 0.5f - 0.5f, 0.f);
+    const int y0 = min((int)sy, H - 1), x0 = min((int)sx, W - 1);
+    const int y1 = min(y0 + 1, H - 1), x1 = min(x0 + 1, W - 1);
+    const float fy = sy - y0, fx = sx - x0;
+    const float4 a = __ldg(p + (size_t)y0 * W + x0), b = __ldg(p + (size_t)y0 * W + x1);
+    const float4 c = __ldg(p + (size_t)y1 * W + x0), d = __ldg(p + (size_t)y1 * W + x1);
+    auto mix = [&](float v00, float v01, float v10, float v11) {
+        return (v00 * (1.f - fx) + v01 * fx) * (1.f - fy) + (v10 * (1.f - fx) + v11 * fx) * fy;
+    };
+    return make_float4(mix(a.x, b.x, c.x, d.x), mix(a.y, b.y, c.y, d.y), mix(a.z, b.z, c.z, d.z), mix(a.w, b.w, c.w, d.w));
+}
+__global__ void __launch_bounds__(128) head_fwd_kernel(const float4* __restrict__ feat4, const float4* __restrict__ base,
+                                                       int rows, int H, int W, float4* __restrict__ out) {
+    const int Ho = 2 * H, Wo = 2 * W;
+    for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
+        const int b = row / Ho, oy = row - b * Ho;
+        const float4* f4 = feat4 + ((size_t)b * H + oy / 2) * W * 4 + 2 * (oy & 1);
+        for (int ox = blockIdx.x * 128 + threadIdx.x; ox < Wo; ox += gridDim.x * 128) {
+            const float4 f = __ldg(f4 + (size_t)(ox >> 1) * 4 + (ox & 1));
+            const float4 u = bilerp_base4(base + (size_t)b * H * W, H, W, oy, ox);
+            out[(size_t)row * Wo + ox] = make_float4(f.x + u.x, f.y + u.y, f.z + u.z, f.w + u.w);
+        }
+    }
+}
+// The same a channel at a time, for pointers that are not on 16 bytes.
+__global__ void head_fwd_unaligned_kernel(const float* feat16, const float* base, int N, int H, int W, float* out) {
     const int Ho = 2 * H, Wo = 2 * W;
     const long long n = (long long)N * Ho * Wo * 4;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
@@ -631,8 +778,17 @@ int vrc_nn_relu_bwd(const void* y, void* dy, long long n, int leaky, void* strea
 
 int vrc_nn_avgpool2(const void* in, int N, int H, int W, int C, float scale, void* out, void* stream) {
     if (H % 2 || W % 2) return 1;
-    avgpool_kernel<<<ew_grid((long long)N * H * W * C / 4), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(in), N, H, W, C, scale, static_cast<__nv_bfloat16*>(out));
+    const int rows = N * (H / 2);
+    const bool wide = C % 8 == 0 && (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
+    const long long per_row = (long long)(W / 2) * (wide ? C / 8 : C);
+    const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>((per_row + 255) / 256, 65535)),
+                    (unsigned)std::max(1, std::min(rows, 65535)));
+    const auto* i = static_cast<const __nv_bfloat16*>(in);
+    auto* o = static_cast<__nv_bfloat16*>(out);
+    if (wide)
+        avgpool_kernel<8><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(i, rows, H, W, C, scale, o);
+    else
+        avgpool_kernel<1><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(i, rows, H, W, C, scale, o);
     return status_of(cudaGetLastError());
 }
 
@@ -656,8 +812,15 @@ int vrc_nn_add(void* a, const void* b, long long n, void* stream) {
 }
 
 int vrc_nn_head_fwd(const float* feat16, const float* base, int N, int H, int W, float* out, void* stream) {
-    head_fwd_kernel<<<ew_grid((long long)N * H * W * 16), 256, 0, static_cast<cudaStream_t>(stream)>>>(feat16, base, N,
-                                                                                                       H, W, out);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int rows = 2 * N * H;
+    if ((reinterpret_cast<uintptr_t>(feat16) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) % 16) {
+        head_fwd_unaligned_kernel<<<ew_grid((long long)N * H * W * 16), 256, 0, st>>>(feat16, base, N, H, W, out);
+    } else {
+        const dim3 grid((unsigned)std::max(1, (2 * W + 127) / 128), (unsigned)std::max(1, std::min(rows, 65535)));
+        head_fwd_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const float4*>(feat16), reinterpret_cast<const float4*>(base),
+                                              rows, H, W, reinterpret_cast<float4*>(out));
+    }
     return status_of(cudaGetLastError());
 }
 
