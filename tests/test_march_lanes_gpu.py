@@ -82,3 +82,38 @@ def test_early_termination_in_a_group(ctx, size, ert):
     b, sb = v.render(ctx, vol16, tf, q, None, None, v.OUT_RGBA32F)
     np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
     assert sa.samples == sb.samples
+
+
+@pytest.mark.parametrize("rate", [0.7, 1.0, 2.0, 3.3])  # steps above and below a voxel: without and with the run rule
+@pytest.mark.parametrize("shade", [0, 1])
+@pytest.mark.parametrize("dtype", [v.U8, v.F32])
+def test_preintegration_lanes_agree(ctx, dtype, shade, rate):
+    """Pre-integration on several lanes a ray, with the queue and on one lane
+    (16^3 bricks): image, auxiliary image, samples, with and without skipping,
+    early termination off and on."""
+    dims = (70, 61, 53)
+    vox = synth.synth_volume(synth.SHELLS, dtype, dims, 77)
+    unit = {v.U8: 255.0, v.F32: 1.0}[dtype]
+    keys = synth.tf_keys_trapezoids([0.25, 0.45, 0.65, 0.8], 3, alpha_range=(0.1, 0.5), top=(0.02, 0.04))
+    vols = [v.Volume(ctx, vox, (0.8, 1.0, 1.1), brick_size=b) for b in (32, 16)]
+    tf = v.TransferFunction(ctx, v.TransferFunction.bake(keys, 1024), (float(vox.min()) / unit, float(vox.max()) / unit))
+    table = v.PreIntegrationTable(ctx, v.PreIntegrationTable.bake_source(keys, 256), v.sampling_step(vols[0], rate))
+    tf.set_preintegration(table)
+    pos, focus, near, far = synth.orbit_camera(dims, (0.8, 1.0, 1.1), 30.0, 20.0, 1.1)
+    for width, height in ((203, 151), (641, 360), (1403, 320)):  # 8 lanes, 4 lanes, queue
+        for skip, ert in ((1, 0.95), (0, 0.95), (1, 1.5), (1, 0.0)):
+            got = []
+            for vol in vols:
+                p = v.default_params(width, height)
+                p.camera = v.make_camera(pos, focus, near=near, far=far)
+                p.light_position[:] = [*pos, 1.0]
+                p.sampling_rate, p.shading, p.ert_threshold = rate, shade, ert
+                p.empty_space_skipping, p.entry_exit_mode = skip, v.EE_ANALYTIC
+                p.classification = v.CLASSIFY_PREINTEGRATED
+                got.append(_render(ctx, vol, tf, p, (0, 0, width, height)))
+            (a, ax, sa), (b, bx, sb) = got
+            np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
+            np.testing.assert_array_equal(ax.view(np.uint32), bx.view(np.uint32))
+            assert sa.samples == sb.samples and (ert == 0.0 or (a[..., 3] > 0).any())
+    tf.close()
+    table.close()

@@ -936,29 +936,36 @@ __device__ __forceinline__ bool empty_cell(const MarchParams& P, const BoxExit& 
 }
 
 // What a ray's samples so far have left; t, loop: the next sample. In the
-// queue of unfinished rays: two float4.
+// queue of unfinished rays: two float4 (pre-integration has no maximum, the
+// other modes no previous sample).
 struct RayState {
     float4 res;
     float max_int, t;
     int loop;
-    bool hit;  // the auxiliary output has the first sample with alpha > 0
+    bool hit;         // the auxiliary output has the first sample with alpha > 0
+    float t_prev;     // pre-integration: the sample before t, and whether its cell was empty
+    bool prev_empty;
     __device__ __forceinline__ void begin(const MarchParams& P) {
         res = make_float4(0.f, 0.f, 0.f, 0.f);
-        max_int = t = 0.f;
+        max_int = t = t_prev = 0.f;
         loop = 0;
         hit = P.aux == nullptr;
+        prev_empty = false;
     }
-    __device__ __forceinline__ void store(float4* q, int pix) const {
+    template <bool PI> __device__ __forceinline__ void store(float4* q, int pix) const {
         q[0] = res;
-        q[1] = make_float4(max_int, t, __int_as_float(loop | (hit ? 1 << 30 : 0)), __int_as_float(pix));
+        q[1] = make_float4(PI ? t_prev : max_int, t, __int_as_float(loop | (hit ? 1 << 30 : 0) | (prev_empty ? 1 << 29 : 0)),
+                           __int_as_float(pix));
     }
-    __device__ __forceinline__ int load(const float4* q) {
+    template <bool PI> __device__ __forceinline__ int load(const float4* q) {
         res = q[0];
         const float4 r = q[1];
-        max_int = r.x;
+        (PI ? t_prev : max_int) = r.x;
         t = r.y;
-        loop = __float_as_int(r.z) & ((1 << 30) - 1);
-        hit = (__float_as_int(r.z) >> 30) != 0;
+        const int bits = __float_as_int(r.z);
+        loop = bits & ((1 << 29) - 1);
+        hit = ((bits >> 30) & 1) != 0;
+        prev_empty = ((bits >> 29) & 1) != 0;
         return __float_as_int(r.w);
     }
 };
@@ -990,8 +997,9 @@ __device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __
     float last = 0.f;  // lastIntensity (cpuraycaster.cpp:235), TF-normalised
     // pre-integration: whether the previous sample lay in an empty cell, and
     // whether `last` still has to be read at t_last (the last skipped sample)
-    bool prev_empty = false, last_stale = false;
-    float t_last = 0.f;
+    bool& prev_empty = st.prev_empty;
+    bool last_stale = false;
+    float& t_last = st.t_prev;
     long long marked = -1;             // last brick recorded as read (cache refinement)
     // POOL: the brick of the last fetched sample and its start (a slot lookup
     // each); a device-resident pool's address is two multiply-adds
@@ -1140,6 +1148,7 @@ __device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __
             res.w = 1.f;
             finished = true;
         }
+        if (PI && STOP) t_last = t;  // where another kernel reads the previous sample
         t = a_(t, step);
         ++loop;
         finished = finished || (t > tend);
@@ -1176,12 +1185,19 @@ __device__ __forceinline__ bool march_ray(const MarchParams& P, const uchar4* __
 // `alive` is the same in a group, and so are f, l, px, py. A ray's chain of
 // dependent loads gets G times shorter where its samples are occupied, for G
 // times the lanes on a run through empty space.
+//
+// Pre-integration: a sample is classified unless it and the one before it lie
+// in empty cells a step of less than a voxel apart (as in march_ray; with
+// longer steps every sample of a pass is), with the TF coordinate of the lane
+// before. The last sample's coordinate goes on to the next pass; where it was
+// not read, or samples were jumped over, lane 0 reads it when it is needed.
 template <int DT, int COMP, int SHADE, int BS, int G>
 __device__ __forceinline__ void march_ray_group(const MarchParams& P, const uchar4* __restrict__ s_tf,
                                                 const float* __restrict__ s_alpha, bool alive, float4 f, float4 l,
                                                 int px, int py, RayState& st, RayCounts& cnt) {
     using T = typename Vox<DT>::T;
     using BG = BrickGeom<BS>;
+    constexpr bool PI = COMP == COMP_DVR_PREINT;
     constexpr bool ERT = !(COMP == VRC_MIP || COMP == VRC_MOP || COMP == VRC_MIDA);
     constexpr unsigned GM = (1u << G) - 1u;
     const T* __restrict__ bricks = reinterpret_cast<const T*>(P.bricks);
@@ -1195,6 +1211,8 @@ __device__ __forceinline__ void march_ray_group(const MarchParams& P, const ucha
     float &max_int = st.max_int, &t = st.t;
     int& loop = st.loop;
     bool& hit = st.hit;
+    float last = 0.f;             // pre-integration: TF coordinate of the sample before t
+    bool stale = PI && loop > 0;  // ... still to be read at st.t_prev
     bool finished = !alive;
     while (__any_sync(FULL, !finished)) {
         // this lane's sample: t advanced `sub` times, as the one-at-a-time loop does
@@ -1207,47 +1225,76 @@ __device__ __forceinline__ void march_ray_group(const MarchParams& P, const ucha
         tn = a_(tn, step);
         const bool valid = !finished && loop + sub < LOOP_CAP && (sub == 0 || !(tl > tend));
         float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-        float rw = 0.f, tsafe = 0.f, gmag2 = 0.f;
+        float rw = 0.f, tsafe = 0.f, gmag2 = 0.f, cur = 0.f;
         bool empty = false;
+        unsigned gval, gemp, gcls, gread;  // per group: valid samples, empty, classified, read
+        SamplePos p;
+        // A sample's voxels and intensity; classify(raw, ...) then colours it
+        // from values still in registers.
+        auto read = [&](auto classify) {
+            const int sh = BG::shift(P.L), S = BG::S(P.L);
+            const int bX = p.ix >> sh, bY = p.iy >> sh, bZ = p.iz >> sh;
+            const T* __restrict__ b = bricks + (long long)((bZ * P.L.nb[1] + bY) * P.L.nb[0] + bX) * BG::stride(P.L);
+            const float fx = s_(p.vx, p.flx), fy = s_(p.vy, p.fly), fz = s_(p.vz, p.flz);
+            const T* __restrict__ vox = b + ((p.iz - (bZ << sh) + APRON_LO) * S + (p.iy - (bY << sh) + APRON_LO)) * S +
+                                        (p.ix - (bX << sh) + APRON_LO);
+            const Raw8 raw = load8<DT>(vox, S, BG::S2(P.L));
+            rw = a_(m_(tri8<DT>(raw, fx, fy, fz), P.rwm_scale), P.rwm_offset);
+            classify(b, vox, raw, fx, fy, fz);
+        };
+        auto shade_sample = [&](const T* b, const T* vox, const Raw8& raw, float fx, float fy, float fz) {
+            if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) {
+                const F3 g = tl == 0.f ? clip_border_gradient(P, F3{p.sx, p.sy, p.sz}, F3{dx, dy, dz}, px, py)
+                                       : central_gradient<DT, BS, false>(P, bricks, b, vox, raw, p, fx, fy, fz);
+                if (!hit) gmag2 = g.x * g.x + g.y * g.y + g.z * g.z;
+                shade(P, p, g, c);
+            }
+        };
         if (valid) {
-            SamplePos p;
             p.set(P, f, dx, dy, dz, tl);
             if (P.occupancy) empty = empty_cell<COMP>(P, bx, f, dx, dy, dz, p, tl, max_int, tsafe);
-            if (!empty) {
-                const int sh = BG::shift(P.L), S = BG::S(P.L);
-                const int bX = p.ix >> sh, bY = p.iy >> sh, bZ = p.iz >> sh;
-                const T* __restrict__ b =
-                    bricks + (long long)((bZ * P.L.nb[1] + bY) * P.L.nb[0] + bX) * BG::stride(P.L);
-                const float fx = s_(p.vx, p.flx), fy = s_(p.vy, p.fly), fz = s_(p.vz, p.flz);
-                const T* __restrict__ vox = b + ((p.iz - (bZ << sh) + APRON_LO) * S + (p.iy - (bY << sh) + APRON_LO)) * S +
-                                            (p.ix - (bX << sh) + APRON_LO);
-                const Raw8 raw = load8<DT>(vox, S, BG::S2(P.L));
-                rw = a_(m_(tri8<DT>(raw, fx, fy, fz), P.rwm_scale), P.rwm_offset);
-                c = tf_colour<false>(P, s_tf, s_alpha, rw);
-                if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) {
-                    const F3 g = tl == 0.f ? clip_border_gradient(P, F3{p.sx, p.sy, p.sz}, F3{dx, dy, dz}, px, py)
-                                           : central_gradient<DT, BS, false>(P, bricks, b, vox, raw, p, fx, fy, fz);
-                    if (!hit) gmag2 = g.x * g.x + g.y * g.y + g.z * g.z;
-                    shade(P, p, g, c);
-                }
+            if (!PI && !empty)
+                read([&](const T* b, const T* vox, const Raw8& raw, float fx, float fy, float fz) {
+                    c = tf_colour<false>(P, s_tf, s_alpha, rw);
+                    shade_sample(b, vox, raw, fx, fy, fz);
+                });
+        }
+        gval = (__ballot_sync(FULL, valid) >> base) & GM, gemp = (__ballot_sync(FULL, empty) >> base) & GM;
+        gcls = gread = gval & ~gemp;
+        if (PI) {
+            gcls = P.pi_chain ? gval & ~(gemp & (gemp << 1 | (st.prev_empty ? 1u : 0u))) : gval;
+            gread = gcls | gcls >> 1;  // the sample before each classified one too
+            if (stale && (gcls & 1u) && sub == 0) {
+                cnt.runs += 0x10000u;
+                const float x = a_(f.x, m_(st.t_prev, dx)), y = a_(f.y, m_(st.t_prev, dy)), z = a_(f.z, m_(st.t_prev, dz));
+                const float v = tap_norm<DT, false>(P, bricks, to_voxel(P, 0, x), to_voxel(P, 1, y), to_voxel(P, 2, z));
+                last = rw_to_tf(a_(m_(v, P.rwm_scale), P.rwm_offset), P.tf_lo, P.tf_hi, P.tf_rcp);
+            }
+            // every lane of the warp takes part in handing the coordinates up,
+            // so the colour is looked up, and shaded from voxels read again,
+            // after it
+            if ((gread >> sub) & 1u)
+                read([&](const T*, const T*, const Raw8&, float, float, float) {
+                    cur = rw_to_tf(rw, P.tf_lo, P.tf_hi, P.tf_rcp);
+                });
+            const float up = __shfl_up_sync(FULL, cur, 1, G);
+            if ((gcls >> sub) & 1u) {
+                c = __ldg(P.pi_table + (size_t)tf_index(cur, P.pi_res) * P.pi_res + tf_index(sub > 0 ? up : last, P.pi_res));
+                if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) read(shade_sample);
             }
         }
-        const unsigned val = __ballot_sync(FULL, valid), emp = __ballot_sync(FULL, empty);
+        const bool reads = (gread >> sub) & 1u;
         const unsigned vis = __ballot_sync(FULL, c.w > 0.f);
-        const unsigned gval = (val >> base) & GM, gfet = gval & ~(emp >> base), gvis = (vis >> base) & GM;
+        const unsigned gvis = (vis >> base) & GM;
         int used = __popc(gval);  // samples of this pass that the ray takes
         bool stop = false;
         if (vis != 0u || (ERT && P.ert <= 0.f)) {
-            if (!hit && gvis) {
-                hit = true;
-                if (sub == __ffs(gvis) - 1) write_aux(P, px, py, tl, tend, gmag2);
-            }
 #pragma unroll
             for (int k = 0; k < G; ++k) {
                 const float4 ck = make_float4(__shfl_sync(FULL, c.x, k, G), __shfl_sync(FULL, c.y, k, G),
                                               __shfl_sync(FULL, c.z, k, G), __shfl_sync(FULL, c.w, k, G));
                 const float rk = COMP == VRC_MIP || COMP == VRC_MIDA ? __shfl_sync(FULL, rw, k, G) : 0.f;
-                if (!stop && ((gfet >> k) & 1u)) {
+                if (!stop && ((gcls >> k) & 1u)) {
                     if ((gvis >> k) & 1u) composite<COMP>(P, res, max_int, ck, rk);
                     if (ERT && res.w >= P.ert) {
                         res.w = 1.f;
@@ -1256,8 +1303,13 @@ __device__ __forceinline__ void march_ray_group(const MarchParams& P, const ucha
                     }
                 }
             }
+            const int first = __ffs(gvis) - 1;  // none: -1
+            if (!hit && first >= 0 && first < used) {
+                hit = true;
+                if (sub == first) write_aux(P, px, py, tl, tend, gmag2);
+            }
         }
-        if (sub < used && ((gfet >> sub) & 1u)) {
+        if (sub < used && reads) {
             ++cnt.fetched_shaded;
             if (SHADE == VRC_SHADE_PHONG && c.w > 0.f) cnt.fetched_shaded += 0x10000u;
         }
@@ -1265,13 +1317,25 @@ __device__ __forceinline__ void march_ray_group(const MarchParams& P, const ucha
         finished = finished || stop || used < G || tn > tend || loop >= LOOP_CAP;
         t = tn;
         const float ts = __shfl_sync(FULL, tsafe, G - 1, G);
-        if (!finished && ((emp >> (base + G - 1)) & 1u)) {
+        if (PI) {
+            last = __shfl_sync(FULL, cur, G - 1, G);
+            st.t_prev = __shfl_sync(FULL, tl, G - 1, G);
+            stale = !(gread >> (G - 1));
+            st.prev_empty = (gemp >> (G - 1)) != 0u;
+        }
+        if (!finished && (gemp >> (G - 1)) != 0u) {
             // the last sample's cell is empty: so are the samples up to its exit
             if (sub == 0) ++cnt.runs;
             const float lim = fminf(ts, tend);
             while (t <= lim && loop < LOOP_CAP) {
-                jump_empty_run(t, loop, step, lim);
+                const int before_jump = loop;
+                jump_empty_run<PI>(t, loop, step, lim, &st.t_prev);
+                if (PI && loop > before_jump) stale = true;
                 if (t <= lim && loop < LOOP_CAP) {
+                    if (PI) {
+                        st.t_prev = t;
+                        stale = true;
+                    }
                     t = a_(t, step);
                     ++loop;
                 }
@@ -1362,7 +1426,7 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_kernel(const 
                 unsigned at = 0;
                 if (lane == 0) at = atomicAdd(P.queue_count, (unsigned)__popc(left));
                 at = __shfl_sync(FULL, at, 0) + __popc(left & ((1u << lane) - 1u));
-                if (!done) st.store(P.queue + 2 * (size_t)at, (int)pix);
+                if (!done) st.store<COMP == COMP_DVR_PREINT>(P.queue + 2 * (size_t)at, (int)pix);
             }
         }
     }
@@ -1400,7 +1464,7 @@ __global__ void __launch_bounds__(256, VRC_MARCH_MIN_BLOCKS) march_group_kernel(
         if (QUEUE) {
             const unsigned q = (unsigned)tile * (32 / G) + ray;
             inside = q < queued;
-            const int pix = inside ? st.load(P.queue + 2 * (size_t)q) : 0;
+            const int pix = inside ? st.load<COMP == COMP_DVR_PREINT>(P.queue + 2 * (size_t)q) : 0;
             py = pix / P.W;
             px = pix - py * P.W;
         } else {
@@ -1523,13 +1587,12 @@ cudaError_t launch_group(const MarchParams& p, int num_sms, cudaStream_t s) {
 // everywhere and the queue only adds to the work (512^3 MIP at 1080p 655 ->
 // 782 us, 1280x720 628 -> 970); they take 4 lanes up to 16,200 tiles (MIP 611
 // -> 394), 2 up to 28,800 (MIP 628 -> 595, MOP 534 -> 405), then one.
-// Pre-integration carries the previous sample along, a brick cache's use
-// marks depend on which samples are read, and first-hit rays end early: one
-// lane.
+// A brick cache's use marks depend on which samples are read, and first-hit
+// rays end early: one lane.
 template <int DT, int COMP, int SHADE, int BS, bool POOL>
 cudaError_t launch_t(const MarchParams& p, int num_sms, cudaStream_t s) {
     const long long tiles = (long long)p.tiles_x * p.tiles_y;
-    constexpr bool ERT = COMP == VRC_DVR || COMP == VRC_ISO;
+    constexpr bool ERT = COMP == VRC_DVR || COMP == VRC_ISO || COMP == COMP_DVR_PREINT;
     constexpr bool ALL = COMP == VRC_MIP || COMP == VRC_MOP || COMP == VRC_MIDA;
     if constexpr (BS == 32 && !POOL && (ERT || ALL)) {
         const long long warps = 24LL * num_sms;
