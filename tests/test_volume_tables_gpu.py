@@ -65,3 +65,29 @@ def test_distance_field_on_any_row_length(ctx, shape, share):
         got = buf.cpu().numpy()
         np.testing.assert_array_equal(got[shift:shift + occ.size].reshape(shape), want)
         assert (got[:shift] == 77).all() and (got[shift + occ.size:] == 77).all()
+
+
+@pytest.mark.parametrize("shape", [(17, 130, 64), (9, 33, 460), (33, 65, 78), (1, 2100, 61), (140, 31, 17), (24, 70, 144)])
+@pytest.mark.parametrize("share", [0.0, 2e-5, 0.002, 1.0])
+def test_distance_field_by_bit_planes(ctx, shape, share):
+    """Maps large enough for the bit planes: rows of whole and partial words,
+    outputs that start on 16 bytes and that do not, every distance up to the cap."""
+    import torch
+    from scipy import ndimage
+    nz, ny, nx = shape
+    occ = np.random.default_rng(nx + ny).random(shape) < share
+    if share == 2e-5:
+        occ[-1, -1, -1] = occ[0, ny // 3, 0] = True
+    want = np.minimum(ndimage.distance_transform_cdt(~occ, "chessboard"), 16) if occ.any() else np.full(shape, 16)
+    flat = np.zeros((occ.size + 31) // 32 * 32, np.uint8)
+    flat[: occ.size] = occ.reshape(-1)
+    bits = torch.from_numpy(np.packbits(flat, bitorder="little").view(np.int32).copy()).cuda()
+    buf = torch.full((occ.size + 16,), 77, dtype=torch.uint8, device="cuda")
+    for shift in (0, 4, 3):
+        buf.fill_(77)
+        torch.cuda.synchronize()
+        assert v.lib().vrc_occupancy_distance(ctx.handle, C.c_void_p(bits.data_ptr()), nx, ny, nz,
+                                              C.c_void_p(buf[shift:].data_ptr())) == 0
+        got = buf.cpu().numpy()
+        np.testing.assert_array_equal(got[shift:shift + occ.size].reshape(shape), want)
+        assert (got[:shift] == 77).all() and (got[shift + occ.size:] == 77).all()

@@ -1232,7 +1232,12 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         VRC_CUDA(ctx, ensure((void**)&ctx->d_occ, &ctx->occ_bytes, vrc::occupancy_bytes(n)));
         if (use_dist) {
             VRC_CUDA(ctx, ensure((void**)&ctx->d_dist, &ctx->dist_bytes, (size_t)n));
-            VRC_CUDA(ctx, ensure((void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes, (size_t)n));
+            // the passes take less scratch where the planes' does not fit
+            if (ensure((void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes,
+                       std::max((size_t)n, vrc::occ_distance_scratch(nc))) != cudaSuccess) {
+                cudaGetLastError();
+                VRC_CUDA(ctx, ensure((void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes, (size_t)n));
+            }
         }
         if (use_coarse)
             VRC_CUDA(ctx, ensure((void**)&ctx->d_occ_coarse, &ctx->occ_coarse_bytes,
@@ -1260,8 +1265,8 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         P.skip_margin = 0.01f + 2e-5f * float(maxdim);
         if (use_dist) {
             if (!cached) {
-                VRC_CUDA(ctx, vrc::launch_occ_distance(ctx->d_occ, nc, ctx->d_dist, ctx->d_dist_tmp, s));
-                occ_launches += 3;
+                VRC_CUDA(ctx, vrc::launch_occ_distance(ctx->d_occ, nc, ctx->d_dist, ctx->d_dist_tmp, ctx->dist_tmp_bytes, s));
+                occ_launches += vrc::occ_distance_launches(nc, ctx->dist_tmp_bytes);
             }
             P.occ_dist = ctx->d_dist;
         }

@@ -227,7 +227,13 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
     cudaStream_t s = ctx->stream;
     if (!occ_jobs.empty()) {
         uint8_t* dist_tmp = nullptr;  // scratch of the distance passes, shared by the requests in turn
-        if ((e = cudaMalloc((void**)&dist_tmp, (size_t)max_cells)) != cudaSuccess) {
+        size_t tmp_bytes = (size_t)max_cells;
+        for (const Occ& j : occ_jobs) tmp_bytes = std::max(tmp_bytes, vrc::occ_distance_scratch(j.nc));
+        if ((e = cudaMalloc((void**)&dist_tmp, tmp_bytes)) != cudaSuccess) {
+            cudaGetLastError();
+            e = cudaMalloc((void**)&dist_tmp, tmp_bytes = (size_t)max_cells);
+        }
+        if (e != cudaSuccess) {
             release(b);
             return bfail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_batch_create: distance scratch allocation");
         }
@@ -236,7 +242,7 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
             if (me == cudaSuccess)
                 me = vrc::launch_occupancy(j.mn, j.mx, j.cells, j.tf->d_prefix, j.tf->width, j.vol->desc.rwm_scale,
                                            j.vol->desc.rwm_offset, j.tf->lo, j.tf->hi, j.map, s);
-            if (me == cudaSuccess) me = vrc::launch_occ_distance(j.map, j.nc, j.dist, dist_tmp, s);
+            if (me == cudaSuccess) me = vrc::launch_occ_distance(j.map, j.nc, j.dist, dist_tmp, tmp_bytes, s);
         }
         if (me == cudaSuccess) me = cudaStreamSynchronize(s);
         cudaFree(dist_tmp);

@@ -2,6 +2,7 @@
 // against (an L2-resident buffer read repeatedly by every SM).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <string>
 
 #include "vrc_internal.h"
@@ -31,9 +32,10 @@ extern "C" vrc_status vrc_occupancy_distance(vrc_context* ctx, const uint32_t* d
     if (n >= (1LL << 32)) return VRC_ERR_INVALID_ARG;
     const int nc[3] = {nx, ny, nz};
     uint8_t* tmp = nullptr;
+    const size_t bytes = std::max((size_t)n, vrc::occ_distance_scratch(nc));
     cudaError_t e = cudaSetDevice(ctx->device);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, (size_t)n);
-    if (e == cudaSuccess) e = vrc::launch_occ_distance(d_bits, nc, d_out, tmp, ctx->stream);
+    if (e == cudaSuccess) e = cudaMalloc(&tmp, bytes);
+    if (e == cudaSuccess) e = vrc::launch_occ_distance(d_bits, nc, d_out, tmp, bytes, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
     if (e != cudaSuccess) {

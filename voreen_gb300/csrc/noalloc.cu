@@ -152,7 +152,7 @@ vrc_status render_noalloc(const vrc_volume* vol, const vrc_tf* tf, const vrc_ren
         // the cells' distance field: an empty run jumps the whole empty box
         // around its cell (MIP's max-based skipping is not taken here)
         uint8_t* dist = scratch + DIST_OFFSET;
-        if ((e = vrc::launch_occ_distance(occ, nc, dist, dist + VRC_NOALLOC_MAX_CELLS, s)) != cudaSuccess)
+        if ((e = vrc::launch_occ_distance(occ, nc, dist, dist + VRC_NOALLOC_MAX_CELLS, VRC_NOALLOC_MAX_CELLS, s)) != cudaSuccess)
             return cuda_status(e);
         P.occ_dist = dist;
         int shift = 0;

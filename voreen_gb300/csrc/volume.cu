@@ -331,7 +331,8 @@ __global__ void __launch_bounds__(256) occupancy_kernel(const float* __restrict_
 // along x the distance to the nearest occupied cell of the row, then along
 // y and along z the min over offsets k of max(|k|, previous pass at c + k).
 // Offsets beyond the cap only give values above it, so each pass looks at
-// |k| < OCC_DIST_CAP. Four cells of a row a thread; a word of four bytes a
+// |k| < OCC_DIST_CAP. Of small maps, where the scratch is short and for caps
+// other than 16 (others: the bit planes below). Four cells of a row a thread; a word of four bytes a
 // load where rows are multiples of four cells (WORDS), else bytes.
 //
 // Along x: the row's bits from 16 below the four cells to 47 above them in one
@@ -437,6 +438,184 @@ __global__ void __launch_bounds__(256) occ_dist_axis_kernel(const uint8_t* __res
         }
     }
 }
+
+// The same map from bit planes, 32 cells a word. The box of radius r around a
+// cell holds an occupied cell or not: one bit, and a cell's distance is the
+// number of radii 0 .. 15 whose bit is 0. The bits of radius r are the occupancy
+// dilated by r along each axis, shifts and ORs of words instead of a min and a
+// max a pair of cells and offset.
+constexpr int DIST_PLANES = 16;
+
+// Word i of row y (cells 32 i ..) with 16 cells on either side as 64 bits: the OR
+// of rows y - r .. y + r takes in two rows a step; along x, a union of shifts by
+// s of a run of c cells each way, s at most 2 c + 1, is one of c + s. A CTA takes
+// 8 words of 32 rows and has their and the 30 rows' windows beside them in shared
+// memory. Planes [r][z][y][i], rows padded to words. Issue slots bound it, some
+// 25 a plane. 512^3 at 2^3 cells: x and y 92 -> 15.5 us (each row's window
+// made anew by each of the 31 threads that take it: 45).
+constexpr int PLANE_WORDS = 8, PLANE_ROWS = 32;
+__global__ void __launch_bounds__(256) occ_planes_xy_kernel(const uint32_t* __restrict__ occ, int nx, int ny, int nz, int tiles_x,
+                                                            int tiles_y, uint32_t* __restrict__ planes) {
+    constexpr int REACH = DIST_PLANES - 1, ROWS = PLANE_ROWS + 2 * REACH;
+    __shared__ unsigned long long win[ROWS][PLANE_WORDS];
+    const int nw = (nx + 31) / 32;
+    const size_t plane = (size_t)nw * ny * nz;
+    const long long last = ((long long)nx * ny * nz + 31) / 32 - 1;
+    const int lane = threadIdx.x % PLANE_WORDS, row = threadIdx.x / PLANE_WORDS;
+    const long long tiles = (long long)tiles_x * tiles_y * nz;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int i = (int)(t % tiles_x) * PLANE_WORDS + lane, y0 = (int)(t / tiles_x % tiles_y) * PLANE_ROWS;
+        const int z = (int)(t / tiles_x / tiles_y), x = i * 32;
+        // beside the row (and, at either end of the map, a clamped word's bits): nothing
+        const unsigned long long mask = (x == 0 ? ~0xffffull : ~0ull) & (nx - x < 48 ? (1ull << (nx - x + 16)) - 1ull : ~0ull);
+        for (int k = row; k < ROWS; k += PLANE_ROWS) {
+            const int y = y0 + k - REACH;
+            unsigned long long v = 0;
+            if (i < nw && (unsigned)y < (unsigned)ny) {
+                const long long s = ((long long)z * ny + y) * nx + x - 16, w = s >> 5;
+                const int sh = (int)(s & 31);
+                const uint32_t a = __ldg(occ + max(w, 0ll)), b = __ldg(occ + min(w + 1, last)), c = __ldg(occ + min(w + 2, last));
+                v = ((unsigned long long)__funnelshift_r(b, c, sh) << 32 | __funnelshift_r(a, b, sh)) & mask;
+            }
+            win[k][lane] = v;
+        }
+        __syncthreads();
+        if (i < nw && y0 + row < ny) {
+            uint32_t* out = planes + ((size_t)z * ny + y0 + row) * nw + i;
+            unsigned long long col = 0;
+#pragma unroll
+            for (int r = 0; r < DIST_PLANES; ++r, out += plane) {
+                col |= win[row + REACH - r][lane] | win[row + REACH + r][lane];
+                unsigned long long v = col;
+#pragma unroll
+                for (int c = 0; c < r;) {
+                    const int s = 2 * c + 1 < r - c ? 2 * c + 1 : r - c;
+                    v |= v << s | v >> s;
+                    c += s;
+                }
+                *out = (uint32_t)(v >> 16);
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Bits i .. i + 3 of w, one to a byte.
+__device__ __forceinline__ uint32_t bits_to_bytes(uint32_t w, int i) {
+    return ((w >> i & 0xfu) * 0x00204081u) & 0x01010101u;
+}
+
+// Along z: a CTA takes 32 words of 8 slices. Warp g ORs the windows of radii g
+// and 15 - g, together the same work for every warp, from the words that the
+// eight windows share and the runs on either side of them; then it takes slice
+// g. A distance's bit s is the parity of the radii r with 2^s dividing r + 1
+// whose bit is 0. Bytes leave 16 at a time, or (WIDE false: rows that are no
+// multiple of 16 cells) by way of shared memory, a word's 32 cells a store.
+// Bound by L2 and by latency. 512^3 at 2^3 cells: z 72 -> 21 us; 500^3: 141 -> 33
+// (all radii one after another in a thread: 33 and 130).
+constexpr int PLANES_Z = 8;
+template <bool WIDE>
+__global__ void __launch_bounds__(256) occ_planes_z_kernel(const uint32_t* __restrict__ planes, int nx, int ny, int nz,
+                                                           uint8_t* __restrict__ out) {
+    __shared__ uint32_t hit[PLANES_Z][DIST_PLANES][32];
+    const unsigned nw = ((unsigned)nx + 31u) / 32u, slice = nw * (unsigned)ny, chunks = (slice + 31u) / 32u;
+    const unsigned tiles = chunks * (((unsigned)nz + PLANES_Z - 1) / PLANES_Z);
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+    for (unsigned t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const unsigned at = t % chunks * 32u + lane;
+        const int z0 = (int)(t / chunks) * PLANES_Z;
+        if (at < slice) {
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                const int r = half ? DIST_PLANES - 1 - g : g;
+                const uint32_t* p = planes + (size_t)r * slice * nz + at;
+                auto word = [&](int z) { return (unsigned)z < (unsigned)nz ? __ldg(p + (size_t)z * slice) : 0u; };
+                uint32_t o[PLANES_Z];
+                if (half || r >= PLANES_Z / 2) {
+                    uint32_t lo[PLANES_Z], hi[PLANES_Z];  // of slices j .. 6, and of 2 r + 1 .. 2 r + j
+#pragma unroll
+                    for (int j = 0; j < PLANES_Z - 1; ++j) {
+                        lo[j] = word(z0 - r + j);
+                        hi[j + 1] = word(z0 + r + 1 + j);
+                    }
+                    uint32_t all = 0;
+#pragma unroll 8
+                    for (int k = PLANES_Z - 1; k <= 2 * r; ++k) all |= word(z0 - r + k);
+                    lo[PLANES_Z - 1] = hi[0] = 0;
+#pragma unroll
+                    for (int j = PLANES_Z - 2; j >= 0; --j) lo[j] |= lo[j + 1];
+#pragma unroll
+                    for (int j = 0; j < PLANES_Z; ++j) {
+                        if (j) hi[j] |= hi[j - 1];
+                        o[j] = all | lo[j] | hi[j];
+                    }
+                } else {  // the windows need not overlap
+#pragma unroll
+                    for (int j = 0; j < PLANES_Z; ++j) o[j] = 0;
+#pragma unroll
+                    for (int k = 0; k < 2 * PLANES_Z - 2; ++k) {
+                        const uint32_t w = k < PLANES_Z + 2 * r ? word(z0 - r + k) : 0u;
+#pragma unroll
+                        for (int j = 0; j < PLANES_Z; ++j)
+                            if (j <= k) o[j] |= k <= j + 2 * r ? w : 0u;
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < PLANES_Z; ++j) hit[j][r][lane] = o[j];
+            }
+        }
+        __syncthreads();
+        const int z = z0 + g;
+        if (z < nz) {
+            uint32_t d[5] = {}, b[8];
+            if (at < slice) {
+#pragma unroll
+                for (int r = 0; r < DIST_PLANES; ++r) {
+                    const uint32_t o = hit[g][r][lane];
+#pragma unroll
+                    for (int s = 0; s < 5; ++s)
+                        if ((r + 1) % (1 << s) == 0) d[s] ^= o;
+                }
+            }
+            d[4] = ~d[4];  // one radius; the others have an even number of them
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                b[i] = 0;
+#pragma unroll
+                for (int s = 0; s < 5; ++s) b[i] += bits_to_bytes(d[s], 4 * i) << s;
+            }
+            uint8_t* q = out + (size_t)z * ny * nx;
+            if (WIDE) {
+                const unsigned y = at / nw;
+                const int x = (int)(at - y * nw) * 32;
+                if (at < slice) {
+                    uint4* q16 = reinterpret_cast<uint4*>(q + (size_t)y * nx + x);
+                    q16[0] = make_uint4(b[0], b[1], b[2], b[3]);
+                    if (nx - x > 16) q16[1] = make_uint4(b[4], b[5], b[6], b[7]);
+                }
+            } else {
+                uint32_t* stage = &hit[g][0][0];  // this warp's slice, read
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) stage[lane * 9 + i] = b[i];
+                __syncwarp();
+                const unsigned first = at - lane, words = min(32u, slice - first);
+                unsigned y = first / nw, i = first - y * nw;
+                for (unsigned k = 0; k < words; ++k) {
+                    const int x = (int)i * 32 + lane;
+                    if (x < nx) q[(size_t)y * nx + x] = reinterpret_cast<const uint8_t*>(stage + k * 9)[lane];
+                    if (++i == nw) { i = 0; ++y; }
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// Maps of fewer words keep the passes: level with them (32^3 cells 9.9 us against
+// 11.3, 48^3 10.5 against 12) and the planes want 64 bytes of scratch a word.
+// 128^3 cells 13 us against 30, 256^3 37 against 164, 250^3 48 against 303.
+constexpr long long PLANES_MIN_WORDS = 4096;
 
 int grid_for(long long n, int block) {
     long long g = (n + block - 1) / block;
@@ -580,7 +759,32 @@ cudaError_t launch_occupancy(const float* bmin, const float* bmax, long long nce
     return cudaGetLastError();
 }
 
-cudaError_t launch_occ_distance(const uint32_t* occ, const int nc[3], uint8_t* dist, uint8_t* tmp, cudaStream_t s) {
+// The planes' words, and whether they gain.
+static long long plane_words(const int nc[3]) { return (long long)((nc[0] + 31) / 32) * nc[1] * nc[2]; }
+size_t occ_distance_scratch(const int nc[3]) {
+    const long long words = plane_words(nc);
+    if (OCC_DIST_CAP != DIST_PLANES || words < PLANES_MIN_WORDS || words >= (1ll << 28)) return 0;
+    return (size_t)words * 4 * DIST_PLANES;
+}
+static bool takes_planes(const int nc[3], size_t tmp_bytes) {
+    const size_t need = occ_distance_scratch(nc);
+    return need && tmp_bytes >= need;
+}
+int occ_distance_launches(const int nc[3], size_t tmp_bytes) { return takes_planes(nc, tmp_bytes) ? 2 : 3; }
+
+cudaError_t launch_occ_distance(const uint32_t* occ, const int nc[3], uint8_t* dist, uint8_t* tmp, size_t tmp_bytes,
+                                cudaStream_t s) {
+    if (takes_planes(nc, tmp_bytes) && reinterpret_cast<uintptr_t>(tmp) % 4 == 0) {
+        uint32_t* planes = reinterpret_cast<uint32_t*>(tmp);
+        const int nw = (nc[0] + 31) / 32, tx = (nw + PLANE_WORDS - 1) / PLANE_WORDS, ty = (nc[1] + PLANE_ROWS - 1) / PLANE_ROWS;
+        occ_planes_xy_kernel<<<grid_for((long long)tx * ty * nc[2], 1), 256, 0, s>>>(occ, nc[0], nc[1], nc[2], tx, ty, planes);
+        const int gz = grid_for(((long long)nw * nc[1] + 31) / 32 * ((nc[2] + PLANES_Z - 1) / PLANES_Z), 1);
+        if ((reinterpret_cast<uintptr_t>(dist) | (uintptr_t)nc[0]) % 16 == 0)
+            occ_planes_z_kernel<true><<<gz, 256, 0, s>>>(planes, nc[0], nc[1], nc[2], dist);
+        else
+            occ_planes_z_kernel<false><<<gz, 256, 0, s>>>(planes, nc[0], nc[1], nc[2], dist);
+        return cudaGetLastError();
+    }
     const int g = grid_for((long long)((nc[0] + 3) / 4) * nc[1] * nc[2], 256);
     const bool words = nc[0] % 4 == 0 && reinterpret_cast<uintptr_t>(dist) % 4 == 0 && reinterpret_cast<uintptr_t>(tmp) % 4 == 0;
     if (words) {

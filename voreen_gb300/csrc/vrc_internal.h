@@ -207,9 +207,14 @@ cudaError_t launch_coarser_minmax(const float* fmin, const float* fmax, const in
 cudaError_t launch_occupancy(const float* bmin, const float* bmax, long long ncells, const int* alpha_prefix,
                              int tf_width, float rwm_scale, float rwm_offset, float tf_lo, float tf_hi,
                              uint32_t* occ, cudaStream_t s);
-// occ_dist from the occupancy bits of an nc[0] x nc[1] x nc[2] cell grid
-// (three separable passes; tmp holds as many bytes as dist).
-cudaError_t launch_occ_distance(const uint32_t* occ, const int nc[3], uint8_t* dist, uint8_t* tmp, cudaStream_t s);
+// occ_dist from the occupancy bits of an nc[0] x nc[1] x nc[2] cell grid. tmp
+// holds at least as many bytes as dist; with occ_distance_scratch of them,
+// maps large enough to gain take the bit planes (volume.cu). The result is the
+// same. occ_distance_launches: the kernels it takes.
+cudaError_t launch_occ_distance(const uint32_t* occ, const int nc[3], uint8_t* dist, uint8_t* tmp, size_t tmp_bytes,
+                                cudaStream_t s);
+size_t occ_distance_scratch(const int nc[3]);
+int occ_distance_launches(const int nc[3], size_t tmp_bytes);
 inline size_t occupancy_bytes(long long ncells) { return (size_t)((ncells + 31) / 32) * 4; }
 
 // Process-unique id of a volume, TF or pre-integration table: identifies
