@@ -9,6 +9,7 @@ import numpy as np
 import pytest
 
 import voreen_gb300 as v
+from voreen_gb300 import synth
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +92,33 @@ def test_distance_field_by_bit_planes(ctx, shape, share):
         got = buf.cpu().numpy()
         np.testing.assert_array_equal(got[shift:shift + occ.size].reshape(shape), want)
         assert (got[:shift] == 77).all() and (got[shift + occ.size:] == 77).all()
+
+
+@pytest.mark.parametrize("dims,dtype,brick", [((2048, 1400, 70), np.uint8, 8), ((1203, 1100, 67), np.uint16, 16),
+                                              ((2501, 1999, 99), np.uint8, 32), ((1024, 640, 131), np.float32, 64)])
+def test_slabs_of_host_voxels_are_the_device_volume(ctx, dims, dtype, brick):
+    """Host voxels come in slabs through a ring of slices, device voxels at
+    once: the same tables and the same image, also from memory that another
+    volume left behind."""
+    import torch
+    rng = np.random.default_rng(dims[0])
+    vox = rng.integers(0, 251, dims[::-1], dtype=np.uint8)
+    vox = {np.uint8: lambda x: x, np.uint16: lambda x: x.astype(np.uint16) * np.uint16(257),
+           np.float32: lambda x: x.astype(np.float32) / np.float32(250)}[dtype](vox)
+    p = v.default_params(96, 64)
+    pos, focus, near, far = synth.orbit_camera(dims, (1.0, 1.0, 1.0), 30.0, 20.0, 1.1)
+    p.camera, p.sampling_rate, p.entry_exit_mode = v.make_camera(pos, focus, near=near, far=far), 0.5, v.EE_ANALYTIC
+    tf = v.TransferFunction(ctx, v.TransferFunction.bake(synth.tf_keys_trapezoids([0.25, 0.65], 3, alpha_range=(0.1, 0.5),
+                                                                                 top=(0.02, 0.04)), 1024), (0.0, 1.0))
+    seen = []
+    for src in (vox, torch.from_numpy(vox).cuda(), vox):
+        vol = v.Volume(ctx, src, brick_size=brick)
+        lo, hi, _ = vol.brick_minmax()
+        image, _ = v.render(ctx, vol, tf, p, out_format=v.OUT_RGBA32F)
+        seen.append((vol.minmax(), np.array(lo), np.array(hi), np.array(image)))
+        vol.close()
+    for got in seen[1:]:
+        assert got[0] == seen[0][0]
+        for a, b in zip(got[1:], seen[0][1:]):
+            np.testing.assert_array_equal(a, b)
+    assert seen[0][3].any()

@@ -16,6 +16,48 @@
 using vrc::BrickLayout;
 using vrc::MarchParams;
 
+namespace vrc {
+
+void* KeptBlock::take(size_t need, size_t* got) {
+    std::lock_guard<std::mutex> g(lock);
+    if (!p || bytes < need || bytes / 2 > need) return nullptr;
+    void* block = p;
+    *got = bytes;
+    p = nullptr;
+    return block;
+}
+
+void KeptBlock::put(void* block, size_t n) {
+    if (n <= VRC_VOLUME_KEEP) {
+        std::lock_guard<std::mutex> g(lock);
+        if (!closed) {
+            std::swap(p, block);
+            bytes = n;
+        }
+    }
+    cudaFree(block);
+}
+
+bool KeptBlock::give_back(bool close) {
+    void* block = nullptr;
+    {
+        std::lock_guard<std::mutex> g(lock);
+        std::swap(p, block);
+        closed = closed || close;
+    }
+    cudaFree(block);
+    return block != nullptr;
+}
+
+cudaError_t device_alloc(KeptBlock& kept, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation || !kept.give_back(false)) return e;
+    cudaGetLastError();
+    return cudaMalloc(p, bytes);
+}
+
+}  // namespace vrc
+
 namespace {
 
 vrc_status fail(vrc_context* ctx, vrc_status s, const std::string& msg) {
@@ -36,12 +78,12 @@ vrc_status cuda_fail(vrc_context* ctx, cudaError_t e, const char* what) {
     } while (0)
 
 // Grow-only device scratch owned by the context.
-cudaError_t ensure(void** p, size_t* cap, size_t need) {
+cudaError_t ensure(vrc_context* c, void** p, size_t* cap, size_t need) {
     if (*cap >= need && *p) return cudaSuccess;
     if (*p) cudaFree(*p);
     *p = nullptr;
     *cap = 0;
-    cudaError_t e = cudaMalloc(p, need);
+    cudaError_t e = vrc::device_alloc(*c->kept, p, need);
     if (e == cudaSuccess) *cap = need;
     return e;
 }
@@ -206,7 +248,7 @@ vrc_status vrc_context_create(int device, vrc_context** out) {
     if (device < 0 || device >= n) return VRC_ERR_INVALID_ARG;
     vrc_context* c = new (std::nothrow) vrc_context();
     if (!c) return VRC_ERR_OUT_OF_MEMORY;
-    c->device = device;
+    c->device = c->kept->device = device;
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) {
         delete c;
@@ -239,6 +281,11 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_occ_coarse);
     cudaFree(c->d_dist);
     cudaFree(c->d_dist_tmp);
+    cudaFree(c->d_stage);
+    c->kept->give_back(true);
+    for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1]})
+        if (ev) cudaEventDestroy(ev);
+    if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     cudaFree(c->d_prefix);
     cudaFree(c->d_queue);
     cudaFree(c->d_counters);
@@ -274,6 +321,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
     vrc_volume* v = new (std::nothrow) vrc_volume();
     if (!v) return fail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: host allocation");
     v->ctx = ctx;
+    v->kept = ctx->kept;
     v->desc = *desc;
     BrickLayout& L = v->L;
     for (int i = 0; i < 3; ++i) {
@@ -293,10 +341,11 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         delete v;
         return fail(ctx, VRC_ERR_UNSUPPORTED, "vrc_volume_upload: more than 2^31 bricks");
     }
-    void* staging = nullptr;
+    void* staging = nullptr;  // a ring of slices too large to keep
     const void* registered = nullptr;  // caller's host voxels registered for direct device reads
     cudaError_t e = cudaSuccess;
     auto cleanup = [&](vrc_status s, const std::string& m) {
+        if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
         cudaStreamSynchronize(ctx->stream);
         if (staging) cudaFree(staging);
         if (registered) cudaHostUnregister(const_cast<void*>(registered));
@@ -310,15 +359,59 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             (e = cudaHostGetDevicePointer(&v->d_bricks, v->h_bricks, 0)) != cudaSuccess)
             return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: host brick pool allocation failed");
         v->host_bytes = brick_bytes;
-    } else if ((e = cudaMalloc(&v->d_bricks, brick_bytes)) != cudaSuccess) {
-        return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: brick pool allocation failed");
     }
-    if ((e = cudaMalloc((void**)&v->d_bmin, L.nbricks() * sizeof(float))) != cudaSuccess ||
-        (e = cudaMalloc((void**)&v->d_bmax, L.nbricks() * sizeof(float))) != cudaSuccess)
-        return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: min/max table allocation failed");
+    // min/max tables: the bricks' and those of finer empty-space cells (2^3, 4^3,
+    // 8^3, 16^3) below the brick size; 2^3 cells (8 bytes of tables per 8
+    // voxels) only up to 2^VRC_CELL2_LOG2_MAX of them. One allocation with
+    // the brick pool.
     v->bytes = (placement == VRC_PLACE_HOST ? 0 : brick_bytes) + 2 * L.nbricks() * sizeof(float);
-    const void* lin = voxels;
-    if (!on_device && placement == VRC_PLACE_HOST) {
+    auto padded = [](long long n) { return (size_t)((n + 63) / 64 * 64); };
+    size_t floats = 2 * padded(L.nbricks());
+    vrc_cell_level* finest = nullptr;
+    for (int li = 0; li < 4; ++li) {
+        const int C = 2 << li;
+        if (C >= brick_size) continue;
+        vrc_cell_level& lv = v->levels[li];
+        for (int i = 0; i < 3; ++i) lv.nc[i] = (desc->dims[i] + C - 1) / C;
+        if (lv.count() >= (1LL << 32) || (C == 2 && lv.count() > (1LL << VRC_CELL2_LOG2_MAX)))
+            continue;  // beyond the march's 32-bit cell index, or the 2^3 table budget
+        lv.C = C;
+        if (!finest) finest = &lv;
+        floats += 2 * padded(lv.count());
+        v->bytes += 2 * lv.count() * sizeof(float);
+    }
+    const size_t pool = placement == VRC_PLACE_HOST ? 0 : (brick_bytes + 255) / 256 * 256;
+    v->block_bytes = pool + floats * sizeof(float);
+    if (!(v->d_block = ctx->kept->take(v->block_bytes, &v->block_bytes)) &&
+        (e = vrc::device_alloc(*ctx->kept, &v->d_block, v->block_bytes)) != cudaSuccess)
+        return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: brick pool and min/max table allocation failed");
+    if (pool) v->d_bricks = v->d_block;
+    float* table = reinterpret_cast<float*>((char*)v->d_block + pool);
+    auto take = [&](long long n) {
+        float* p = table;
+        table += padded(n);
+        return p;
+    };
+    v->d_bmin = take(L.nbricks());
+    v->d_bmax = take(L.nbricks());
+    for (auto& lv : v->levels)
+        if (lv.C) {
+            lv.d_min = take(lv.count());
+            lv.d_max = take(lv.count());
+        }
+    // bricks and finest cells of brick layers [l0, l1), whose slices are in `lin`
+    auto ingest = [&](const vrc::Slices& lin, int l0, int l1) {
+        cudaError_t r = vrc::launch_brick_build(lin, desc->dtype, L, l0, l1, v->d_bricks, ctx->stream);
+        if (r == cudaSuccess && finest) {
+            const int per = L.B / finest->C;
+            r = vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, finest->C, l0 * per, std::min(l1 * per, finest->nc[2]),
+                                        finest->d_min, finest->d_max, ctx->stream);
+        }
+        return r;
+    };
+    if (on_device) {
+        e = ingest({voxels}, 0, L.nb[2]);
+    } else if (placement == VRC_PLACE_HOST) {
         // no device copy of the linear volume either: the bricking kernels read
         // the caller's voxels through a mapped registration
         void* dp = nullptr;
@@ -327,40 +420,60 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         registered = voxels;
         if ((e = cudaHostGetDevicePointer(&dp, const_cast<void*>(voxels), 0)) != cudaSuccess)
             return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: mapped address: ") + cudaGetErrorString(e));
-        lin = dp;
-    } else if (!on_device) {
-        if ((e = cudaMalloc(&staging, nvox * bpv)) != cudaSuccess)
-            return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: staging allocation failed");
-        if ((e = cudaMemcpyAsync(staging, voxels, nvox * bpv, cudaMemcpyHostToDevice, ctx->stream)) != cudaSuccess)
-            return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: copy: ") + cudaGetErrorString(e));
-        lin = staging;
-    }
-    if ((e = vrc::launch_brick_build(lin, desc->dtype, L, v->d_bricks, ctx->stream)) != cudaSuccess)
-        return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: kernel: ") + cudaGetErrorString(e));
-    // finer empty-space cells (2^3, 4^3, 8^3, 16^3) below the brick size;
-    // 2^3 cells (8 bytes of tables per 8 voxels) only up to
-    // 2^VRC_CELL2_LOG2_MAX of them
-    for (int li = 0; li < 4; ++li) {
-        const int C = 2 << li;
-        if (C >= brick_size) continue;
-        vrc_cell_level& lv = v->levels[li];
-        lv.C = C;
-        for (int i = 0; i < 3; ++i) lv.nc[i] = (desc->dims[i] + C - 1) / C;
-        if (lv.count() >= (1LL << 32) || (C == 2 && lv.count() > (1LL << VRC_CELL2_LOG2_MAX))) {
-            lv.C = 0;  // beyond the march's 32-bit cell index, or the 2^3 table budget
-            continue;
+        e = ingest({dp}, 0, L.nb[2]);
+    } else {
+        // Slabs of whole brick layers through a ring of slices: the bricks and
+        // cells of one are built while the next is copied. The link from the
+        // host bounds it: 512^3 u16 of pageable memory 1500 us at 180 GB/s,
+        // the call 1750 (the kernels' 260 and the allocation and release of a
+        // staged volume, 280, came on top). Slabs of 16 MB 2130 (each copy
+        // returns late), of 33 MB 1790, of 67 MB 1730, one of 268 MB 1820.
+        const size_t slice = (size_t)desc->dims[0] * desc->dims[1] * bpv;
+        const int Z = desc->dims[2];
+        const int layers = (int)std::min<size_t>(std::max<size_t>(VRC_SLAB_BYTES / (slice * L.B), 1), L.nb[2]);
+        const int ring = (int)std::min<long long>(2ll * layers * L.B + vrc::APRON_LO + vrc::APRON_HI, Z);
+        char* stage = nullptr;
+        if (ring * slice <= VRC_STAGE_KEEP) {
+            e = ensure(ctx, &ctx->d_stage, &ctx->stage_bytes, ring * slice);
+            stage = (char*)ctx->d_stage;
+        } else {
+            e = vrc::device_alloc(*ctx->kept, &staging, ring * slice);
+            stage = (char*)staging;
         }
-        if ((e = cudaMalloc((void**)&lv.d_min, lv.count() * sizeof(float))) != cudaSuccess ||
-            (e = cudaMalloc((void**)&lv.d_max, lv.count() * sizeof(float))) != cudaSuccess)
-            return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: cell table allocation failed");
-        v->bytes += 2 * lv.count() * sizeof(float);
-        // the finest level from the voxels, the others each from the one below
-        const vrc_cell_level* fine = li > 0 && v->levels[li - 1].d_max ? &v->levels[li - 1] : nullptr;
-        e = fine ? vrc::launch_coarser_minmax(fine->d_min, fine->d_max, fine->nc, 2, lv.nc, lv.d_min, lv.d_max, ctx->stream)
-                 : vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, C, lv.d_min, lv.d_max, ctx->stream);
-        if (e != cudaSuccess)
-            return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: cell kernel: ") + cudaGetErrorString(e));
+        if (e != cudaSuccess) return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: staging allocation failed");
+        if (!ctx->copy_stream) {
+            e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
+            for (cudaEvent_t* ev : {&ctx->copied[0], &ctx->copied[1], &ctx->consumed[0], &ctx->consumed[1]})
+                if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        }
+        int have = 0;  // slices copied
+        for (int l0 = 0, k = 0; l0 < L.nb[2] && e == cudaSuccess; l0 += layers, k ^= 1) {
+            const int l1 = std::min(l0 + layers, L.nb[2]);
+            const int first = std::max(l0 * L.B - vrc::APRON_LO, 0), end = (int)std::min<long long>((long long)l1 * L.B + vrc::APRON_HI, Z);
+            // the slices this slab brings take the place of those before the last one's
+            if (l0 >= 2 * layers) e = cudaStreamWaitEvent(ctx->copy_stream, ctx->consumed[k], 0);
+            while (have < end && e == cudaSuccess) {
+                const int at = have % ring, n = std::min(end - have, ring - at);
+                e = cudaMemcpyAsync(stage + at * slice, (const char*)voxels + have * slice, n * slice, cudaMemcpyHostToDevice,
+                                    ctx->copy_stream);
+                have += n;
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->copied[k], ctx->copy_stream);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->copied[k], 0);
+            if (e != cudaSuccess)
+                return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: copy: ") + cudaGetErrorString(e));
+            e = ingest({stage, first, first % ring, ring}, l0, l1);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->consumed[k], ctx->stream);
+        }
     }
+    // the coarser levels each from the one below
+    for (int li = 1; li < 4 && e == cudaSuccess; ++li) {
+        vrc_cell_level &lv = v->levels[li], &fine = v->levels[li - 1];
+        if (lv.d_max && fine.d_max)
+            e = vrc::launch_coarser_minmax(fine.d_min, fine.d_max, fine.nc, 2, lv.nc, lv.d_min, lv.d_max, ctx->stream);
+    }
+    if (e != cudaSuccess)
+        return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: kernel: ") + cudaGetErrorString(e));
     // the bricks' from the coarsest cells (half a brick, or a quarter of a 64^3 one)
     const vrc_cell_level* half = nullptr;
     for (const auto& lv : v->levels)
@@ -389,11 +502,13 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
 
 vrc_status vrc_volume_destroy(vrc_volume* v) {
     if (!v) return VRC_ERR_INVALID_ARG;
-    if (v->ctx) cudaSetDevice(v->ctx->device);
-    if (v->h_bricks)
-        cudaFreeHost(v->h_bricks);
+    if (v->kept) cudaSetDevice(v->kept->device);
+    // no frame on any stream reads the volume any more, as after a cudaFree
+    if (v->d_block && v->kept && cudaDeviceSynchronize() == cudaSuccess)
+        v->kept->put(v->d_block, v->block_bytes);
     else
-        cudaFree(v->d_bricks);
+        cudaFree(v->d_block);
+    if (v->h_bricks) cudaFreeHost(v->h_bricks);
     cudaFree(v->d_cache);
     cudaFree(v->d_slot);
     cudaFree(v->d_occ_brick);
@@ -401,12 +516,6 @@ vrc_status vrc_volume_destroy(vrc_volume* v) {
     cudaFree(v->d_cache_dst);
     cudaFree(v->d_used);
     cudaFree(v->d_lod);
-    cudaFree(v->d_bmin);
-    cudaFree(v->d_bmax);
-    for (auto& lv : v->levels) {
-        cudaFree(lv.d_min);
-        cudaFree(lv.d_max);
-    }
     delete v;
     return VRC_OK;
 }
@@ -518,10 +627,10 @@ vrc_status vrc_volume_set_lod(vrc_volume* v, int level) {
             const size_t n1 = (size_t)H.dims[0] * H.dims[1] * H.dims[2];
             void* lin = nullptr;
             void* bricks = nullptr;
-            e = cudaMalloc(&lin, n1 * bpv);
-            if (e == cudaSuccess) e = cudaMalloc(&bricks, (size_t)H.nbricks() * H.brick_stride * bpv);
+            e = vrc::device_alloc(*ctx->kept, &lin, n1 * bpv);
+            if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &bricks, (size_t)H.nbricks() * H.brick_stride * bpv);
             if (e == cudaSuccess) e = vrc::launch_half_sample(src, v->desc.dtype, srcL, H.dims, lin, ctx->stream);
-            if (e == cudaSuccess) e = vrc::launch_brick_build(lin, v->desc.dtype, H, bricks, ctx->stream);
+            if (e == cudaSuccess) e = vrc::launch_brick_build({lin}, v->desc.dtype, H, 0, H.nb[2], bricks, ctx->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
             cudaFree(lin);
             cudaFree(prev);
@@ -967,7 +1076,7 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
                 vol->h_slot_brick.clear();
                 vol->free_slots.clear();
                 std::fill(vol->h_slot.begin(), vol->h_slot.end(), -1);
-                cudaError_t e = cudaMalloc(&vol->d_cache, (size_t)slots * brick_bytes);
+                cudaError_t e = vrc::device_alloc(*ctx->kept, &vol->d_cache, (size_t)slots * brick_bytes);
                 if (e == cudaSuccess) e = cudaMalloc((void**)&vol->d_cache_ids, (size_t)slots * sizeof(long long));
                 if (e == cudaSuccess) e = cudaMalloc((void**)&vol->d_cache_dst, (size_t)slots * sizeof(long long));
                 if (e != cudaSuccess) {
@@ -1166,7 +1275,7 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
             P.entry = reinterpret_cast<const float4*>(me);
             P.exitp = reinterpret_cast<const float4*>(mx);
         } else {
-            VRC_CUDA(ctx, ensure(&ctx->d_ee, &ctx->ee_bytes, 2 * npix * sizeof(float4)));
+            VRC_CUDA(ctx, ensure(ctx, &ctx->d_ee, &ctx->ee_bytes, 2 * npix * sizeof(float4)));
             float4* d = reinterpret_cast<float4*>(ctx->d_ee);
             VRC_CUDA(ctx, cudaMemcpyAsync(d, entry, npix * sizeof(float4), cudaMemcpyHostToDevice, s));
             VRC_CUDA(ctx, cudaMemcpyAsync(d + npix, exitp, npix * sizeof(float4), cudaMemcpyHostToDevice, s));
@@ -1181,7 +1290,7 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
     } else if (mout) {
         P.out = mout;
     } else {
-        VRC_CUDA(ctx, ensure(&ctx->d_out, &ctx->out_bytes, npix * px_bytes));
+        VRC_CUDA(ctx, ensure(ctx, &ctx->d_out, &ctx->out_bytes, npix * px_bytes));
         P.out = ctx->d_out;
     }
     P.out_format = out_format;
@@ -1229,18 +1338,18 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         const uint32_t* occ_before = ctx->d_occ;
         const uint32_t* coarse_before = ctx->d_occ_coarse;
         const uint8_t* dist_before = ctx->d_dist;
-        VRC_CUDA(ctx, ensure((void**)&ctx->d_occ, &ctx->occ_bytes, vrc::occupancy_bytes(n)));
+        VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_occ, &ctx->occ_bytes, vrc::occupancy_bytes(n)));
         if (use_dist) {
-            VRC_CUDA(ctx, ensure((void**)&ctx->d_dist, &ctx->dist_bytes, (size_t)n));
+            VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_dist, &ctx->dist_bytes, (size_t)n));
             // the passes take less scratch where the planes' does not fit
-            if (ensure((void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes,
+            if (ensure(ctx, (void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes,
                        std::max((size_t)n, vrc::occ_distance_scratch(nc))) != cudaSuccess) {
                 cudaGetLastError();
-                VRC_CUDA(ctx, ensure((void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes, (size_t)n));
+                VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes, (size_t)n));
             }
         }
         if (use_coarse)
-            VRC_CUDA(ctx, ensure((void**)&ctx->d_occ_coarse, &ctx->occ_coarse_bytes,
+            VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_occ_coarse, &ctx->occ_coarse_bytes,
                                  vrc::occupancy_bytes(vol->L.nbricks())));
         const bool cached = std::memcmp(key, ctx->occ_key, sizeof(key)) == 0 && ctx->d_occ == occ_before &&
                             (!use_coarse || ctx->d_occ_coarse == coarse_before) &&
@@ -1351,7 +1460,7 @@ vrc_status vrc_entry_exit(vrc_context* ctx, const vrc_volume* vol, const vrc_ren
     const size_t npix = (size_t)p->width * p->height;
     float4 *de = reinterpret_cast<float4*>(entry), *dx = reinterpret_cast<float4*>(exitp);
     if (!out_on_device) {
-        VRC_CUDA(ctx, ensure(&ctx->d_ee, &ctx->ee_bytes, 2 * npix * sizeof(float4)));
+        VRC_CUDA(ctx, ensure(ctx, &ctx->d_ee, &ctx->ee_bytes, 2 * npix * sizeof(float4)));
         de = reinterpret_cast<float4*>(ctx->d_ee);
         dx = de + npix;
     }

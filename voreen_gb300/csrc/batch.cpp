@@ -168,8 +168,8 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
             const long long cells = (long long)nc[0] * nc[1] * nc[2];
             uint32_t* map = nullptr;
             uint8_t* dist = nullptr;
-            if ((e = cudaMalloc((void**)&map, vrc::occupancy_bytes(cells))) == cudaSuccess) b->occ.push_back(map);
-            if (e == cudaSuccess && (e = cudaMalloc((void**)&dist, (size_t)cells)) == cudaSuccess) b->dist.push_back(dist);
+            if ((e = vrc::device_alloc(*ctx->kept, (void**)&map, vrc::occupancy_bytes(cells))) == cudaSuccess) b->occ.push_back(map);
+            if (e == cudaSuccess && (e = vrc::device_alloc(*ctx->kept, (void**)&dist, (size_t)cells)) == cudaSuccess) b->dist.push_back(dist);
             if (e != cudaSuccess) {
                 release(b);
                 return bfail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_batch_create: occupancy allocation");
@@ -229,9 +229,9 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
         uint8_t* dist_tmp = nullptr;  // scratch of the distance passes, shared by the requests in turn
         size_t tmp_bytes = (size_t)max_cells;
         for (const Occ& j : occ_jobs) tmp_bytes = std::max(tmp_bytes, vrc::occ_distance_scratch(j.nc));
-        if ((e = cudaMalloc((void**)&dist_tmp, tmp_bytes)) != cudaSuccess) {
+        if ((e = vrc::device_alloc(*ctx->kept, (void**)&dist_tmp, tmp_bytes)) != cudaSuccess) {
             cudaGetLastError();
-            e = cudaMalloc((void**)&dist_tmp, tmp_bytes = (size_t)max_cells);
+            e = vrc::device_alloc(*ctx->kept, (void**)&dist_tmp, tmp_bytes = (size_t)max_cells);
         }
         if (e != cudaSuccess) {
             release(b);

@@ -21,20 +21,33 @@ namespace {
 // arithmetic: two 64-bit divisions and a store per voxel. The edge is
 // compile-time, so a position in the brick divides by constants, and four
 // consecutive voxels span at most two rows. 512^3 u16: 1095 -> 177 us (the floor at the copy rate: 91).
+template <typename T> struct SlicesOf {
+    const T* base;
+    int first, at, ring;
+    explicit SlicesOf(const Slices& s) : base((const T*)s.base), first(s.first), at(s.at), ring(s.ring) {}
+    // row y of slice z
+    __device__ __forceinline__ const T* row(int z, int y, int X, int Y) const {
+        int i = z - first + at;
+        if (i >= ring) i -= ring;
+        return base + ((long long)i * Y + y) * X;
+    }
+};
+
 template <typename T, int B>
-__global__ void __launch_bounds__(256) brick_build_kernel(const T* __restrict__ lin, BrickLayout L, T* __restrict__ bricks) {
+__global__ void __launch_bounds__(256) brick_build_kernel(SlicesOf<T> lin, BrickLayout L, long long b0, long long b1,
+                                                          T* __restrict__ bricks) {
     constexpr int S = B + APRON_LO + APRON_HI, S2 = S * S, S3 = S2 * S;
     struct alignas(4 * sizeof(T)) Quad {
         T v[4];
     };
     const int X1 = L.dims[0] - 1, Y1 = L.dims[1] - 1, Z1 = L.dims[2] - 1;
-    for (long long b = blockIdx.x; b < L.nbricks(); b += gridDim.x) {
+    for (long long b = b0 + blockIdx.x; b < b1; b += gridDim.x) {
         const unsigned bu = (unsigned)b, nb0 = (unsigned)L.nb[0], nb1 = (unsigned)L.nb[1];  // fewer than 2^31 bricks
         const int x0 = (int)(bu % nb0) * B - APRON_LO, y0 = (int)(bu / nb0 % nb1) * B - APRON_LO,
                   z0 = (int)(bu / nb0 / nb1) * B - APRON_LO;
         T* out = bricks + b * L.brick_stride;
         auto row = [&](int y, int z) {
-            return lin + ((long long)min(max(z0 + z, 0), Z1) * L.dims[1] + min(max(y0 + y, 0), Y1)) * L.dims[0];
+            return lin.row(min(max(z0 + z, 0), Z1), min(max(y0 + y, 0), Y1), L.dims[0], L.dims[1]);
         };
         // the last quad may reach past S^3 into the brick's padding (the stride is a multiple of 64)
         for (int i = threadIdx.x; i < (S3 + 3) / 4; i += 256) {
@@ -135,9 +148,9 @@ __global__ void brick_minmax_kernel(const T* __restrict__ bricks, BrickLayout L,
 // high side of every axis (clamped), i.e. the trilinear support of all
 // samples whose floor voxel lies in the cell. Any cell edge and row length.
 template <typename T>
-__global__ void cell_minmax_kernel(const T* __restrict__ lin, int X, int Y, int Z, int C, int ncx, int ncy,
-                                   long long ncells, float norm, float* cmin, float* cmax) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < ncells;
+__global__ void cell_minmax_kernel(SlicesOf<T> lin, int X, int Y, int Z, int C, int ncx, int ncy, long long c0,
+                                   long long c1, float norm, float* cmin, float* cmax) {
+    for (long long c = c0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; c < c1;
          c += (long long)gridDim.x * blockDim.x) {
         const int cx = (int)(c % ncx), cy = (int)((c / ncx) % ncy), cz = (int)(c / ((long long)ncx * ncy));
         const int x0 = cx * C, y0 = cy * C, z0 = cz * C;
@@ -145,7 +158,7 @@ __global__ void cell_minmax_kernel(const T* __restrict__ lin, int X, int Y, int 
         float mn = INFINITY, mx = -INFINITY;
         for (int z = z0; z <= z1; ++z)
             for (int y = y0; y <= y1; ++y) {
-                const T* row = lin + ((long long)z * Y + y) * X;
+                const T* row = lin.row(z, y, X, Y);
                 for (int x = x0; x <= x1; ++x) {
                     const float v = raw_to_float(row[x]);
                     mn = fminf(mn, v);
@@ -219,11 +232,11 @@ template <> struct Run9<float> {
 // a row, integers compared as pairs. HBM is the bound (the volume read, two
 // floats a cell written). 512^3 u16: 480 -> 82 us (floor: 59).
 template <typename T>
-__global__ void __launch_bounds__(256) cell2_minmax_kernel(const T* __restrict__ lin, int X, int Y, int Z, int ncy,
-                                                           unsigned ngroups, float norm, float* __restrict__ cmin,
+__global__ void __launch_bounds__(256) cell2_minmax_kernel(SlicesOf<T> lin, int X, int Y, int Z, int ncy, unsigned g0,
+                                                           unsigned g1, float norm, float* __restrict__ cmin,
                                                            float* __restrict__ cmax) {
     const unsigned gx = (unsigned)X / 8u;
-    for (unsigned long long i = blockIdx.x * 256ull + threadIdx.x; i < ngroups; i += gridDim.x * 256ull) {
+    for (unsigned long long i = g0 + blockIdx.x * 256ull + threadIdx.x; i < g1; i += gridDim.x * 256ull) {
         const unsigned r = (unsigned)i / gx;
         const int x0 = (int)((unsigned)i - r * gx) * 8, y0 = 2 * (int)(r % (unsigned)ncy), z0 = 2 * (int)(r / (unsigned)ncy);
         const int x8 = min(x0 + 8, X - 1);
@@ -233,7 +246,7 @@ __global__ void __launch_bounds__(256) cell2_minmax_kernel(const T* __restrict__
         for (int dz = 0; dz < 3; ++dz)
 #pragma unroll
             for (int dy = 0; dy < 3; ++dy)
-                run.add(lin + ((long long)min(z0 + dz, Z - 1) * Y + min(y0 + dy, Y - 1)) * X, x0, x8);
+                run.add(lin.row(min(z0 + dz, Z - 1), min(y0 + dy, Y - 1), X, Y), x0, x8);
         float4 mn = make_float4(run.lo(0), run.lo(1), run.lo(2), run.lo(3));
         float4 mx = make_float4(run.hi(0), run.hi(1), run.hi(2), run.hi(3));
         if (norm > 0.f) {
@@ -654,23 +667,26 @@ cudaError_t launch_brick_gather(const void* pool, const long long* ids, const lo
 }
 
 template <typename T>
-static cudaError_t brick_build_t(const T* lin, const BrickLayout& L, T* bricks, cudaStream_t s) {
-    const unsigned g = (unsigned)std::min<long long>(L.nbricks(), 1 << 20);
+static cudaError_t brick_build_t(const Slices& lin, const BrickLayout& L, int layer0, int layer1, T* bricks, cudaStream_t s) {
+    const SlicesOf<T> v(lin);
+    const long long layer = (long long)L.nb[0] * L.nb[1], b0 = layer0 * layer, b1 = layer1 * layer;
+    const unsigned g = (unsigned)std::min<long long>(b1 - b0, 1 << 20);
     switch (L.B) {
-        case 8: brick_build_kernel<T, 8><<<g, 256, 0, s>>>(lin, L, bricks); break;
-        case 16: brick_build_kernel<T, 16><<<g, 256, 0, s>>>(lin, L, bricks); break;
-        case 32: brick_build_kernel<T, 32><<<g, 256, 0, s>>>(lin, L, bricks); break;
-        case 64: brick_build_kernel<T, 64><<<g, 256, 0, s>>>(lin, L, bricks); break;
+        case 8: brick_build_kernel<T, 8><<<g, 256, 0, s>>>(v, L, b0, b1, bricks); break;
+        case 16: brick_build_kernel<T, 16><<<g, 256, 0, s>>>(v, L, b0, b1, bricks); break;
+        case 32: brick_build_kernel<T, 32><<<g, 256, 0, s>>>(v, L, b0, b1, bricks); break;
+        case 64: brick_build_kernel<T, 64><<<g, 256, 0, s>>>(v, L, b0, b1, bricks); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_brick_build(const void* linear, int dtype, const BrickLayout& L, void* bricks, cudaStream_t s) {
+cudaError_t launch_brick_build(const Slices& linear, int dtype, const BrickLayout& L, int layer0, int layer1, void* bricks,
+                               cudaStream_t s) {
     switch (dtype) {
-        case VRC_U8: return brick_build_t((const uint8_t*)linear, L, (uint8_t*)bricks, s);
-        case VRC_U16: return brick_build_t((const uint16_t*)linear, L, (uint16_t*)bricks, s);
-        default: return brick_build_t((const float*)linear, L, (float*)bricks, s);
+        case VRC_U8: return brick_build_t(linear, L, layer0, layer1, (uint8_t*)bricks, s);
+        case VRC_U16: return brick_build_t(linear, L, layer0, layer1, (uint16_t*)bricks, s);
+        default: return brick_build_t(linear, L, layer0, layer1, (float*)bricks, s);
     }
 }
 
@@ -715,25 +731,25 @@ cudaError_t launch_brick_minmax(const void* bricks, int dtype, const BrickLayout
 }
 
 template <typename T>
-static cudaError_t cell_minmax_t(const T* lin, const int d[3], int C, float norm, float* cmin, float* cmax, cudaStream_t s) {
-    const int ncx = (d[0] + C - 1) / C, ncy = (d[1] + C - 1) / C, ncz = (d[2] + C - 1) / C;
-    const long long n = (long long)ncx * ncy * ncz;
-    if (C == 2 && d[0] % 8 == 0 && reinterpret_cast<uintptr_t>(lin) % 16 == 0) {
-        const long long groups = n / 4;
-        cell2_minmax_kernel<T><<<grid_for(groups, 256), 256, 0, s>>>(lin, d[0], d[1], d[2], ncy, (unsigned)groups, norm,
-                                                                     cmin, cmax);
-    } else {
-        cell_minmax_kernel<T><<<grid_for(n, 128), 128, 0, s>>>(lin, d[0], d[1], d[2], C, ncx, ncy, n, norm, cmin, cmax);
-    }
+static cudaError_t cell_minmax_t(const Slices& lin, const int d[3], int C, int cz0, int cz1, float norm, float* cmin,
+                                 float* cmax, cudaStream_t s) {
+    const int ncx = (d[0] + C - 1) / C, ncy = (d[1] + C - 1) / C;
+    const long long layer = (long long)ncx * ncy, c0 = cz0 * layer, c1 = cz1 * layer;
+    const SlicesOf<T> v(lin);
+    if (C == 2 && d[0] % 8 == 0 && reinterpret_cast<uintptr_t>(lin.base) % 16 == 0)
+        cell2_minmax_kernel<T><<<grid_for((c1 - c0) / 4, 256), 256, 0, s>>>(v, d[0], d[1], d[2], ncy, (unsigned)(c0 / 4),
+                                                                            (unsigned)(c1 / 4), norm, cmin, cmax);
+    else
+        cell_minmax_kernel<T><<<grid_for(c1 - c0, 128), 128, 0, s>>>(v, d[0], d[1], d[2], C, ncx, ncy, c0, c1, norm, cmin, cmax);
     return cudaGetLastError();
 }
 
-cudaError_t launch_cell_minmax(const void* linear, int dtype, const int d[3], int C, float* cmin, float* cmax,
-                               cudaStream_t s) {
+cudaError_t launch_cell_minmax(const Slices& linear, int dtype, const int d[3], int C, int cz0, int cz1, float* cmin,
+                               float* cmax, cudaStream_t s) {
     switch (dtype) {
-        case VRC_U8: return cell_minmax_t((const uint8_t*)linear, d, C, 255.f, cmin, cmax, s);
-        case VRC_U16: return cell_minmax_t((const uint16_t*)linear, d, C, 65535.f, cmin, cmax, s);
-        default: return cell_minmax_t((const float*)linear, d, C, 0.f, cmin, cmax, s);
+        case VRC_U8: return cell_minmax_t<uint8_t>(linear, d, C, cz0, cz1, 255.f, cmin, cmax, s);
+        case VRC_U16: return cell_minmax_t<uint16_t>(linear, d, C, cz0, cz1, 65535.f, cmin, cmax, s);
+        default: return cell_minmax_t<float>(linear, d, C, cz0, cz1, 0.f, cmin, cmax, s);
     }
 }
 

@@ -5,6 +5,8 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <memory>
+#include <mutex>
 #include <map>
 #include <string>
 #include <utility>
@@ -187,7 +189,15 @@ cudaError_t launch_march_batch(const BatchReq* reqs, int nreq, const unsigned* t
 // each), i in [0, n).
 cudaError_t launch_brick_gather(const void* pool, const long long* ids, const long long* dst, long long n,
                                 size_t brick_stride_bytes, void* cache, cudaStream_t s);
-cudaError_t launch_brick_build(const void* linear, int dtype, const BrickLayout& L, void* bricks, cudaStream_t s);
+// Slices of a linear volume: all of them, or those of a slab in a ring of
+// `ring` slices that holds slice `first` at `at`.
+struct Slices {
+    const void* base;
+    int first = 0, at = 0, ring = 0x7fffffff;
+};
+// The bricks of layers [layer0, layer1) along z (their voxels and apron).
+cudaError_t launch_brick_build(const Slices& linear, int dtype, const BrickLayout& L, int layer0, int layer1, void* bricks,
+                               cudaStream_t s);
 // Half-resolution linear volume from a bricked one: voxel (x, y, z) = mean of
 // the full-resolution voxels 2x..2x+1 (clamped to the volume) on each axis;
 // integers summed exactly and divided by 8 with truncation.
@@ -196,9 +206,10 @@ cudaError_t launch_half_sample(const void* bricks, int dtype, const BrickLayout&
 cudaError_t launch_brick_minmax(const void* bricks, int dtype, const BrickLayout& L, float* bmin, float* bmax,
                                 cudaStream_t s);
 // Min/max of normalised intensity per cell of edge C over the cell's voxels
-// plus one voxel on the high side (clamped), from the linear volume.
-cudaError_t launch_cell_minmax(const void* linear, int dtype, const int dims[3], int C, float* cmin, float* cmax,
-                               cudaStream_t s);
+// plus one voxel on the high side (clamped), from the linear volume; cells
+// [cz0, cz1) along z.
+cudaError_t launch_cell_minmax(const Slices& linear, int dtype, const int dims[3], int C, int cz0, int cz1, float* cmin,
+                               float* cmax, cudaStream_t s);
 // The same for cells of `factor` (2 or 4) times the edge, from a level's own.
 cudaError_t launch_coarser_minmax(const float* fmin, const float* fmax, const int fnc[3], int factor, const int nc[3],
                                   float* cmin, float* cmax, cudaStream_t s);
@@ -216,6 +227,25 @@ cudaError_t launch_occ_distance(const uint32_t* occ, const int nc[3], uint8_t* d
 size_t occ_distance_scratch(const int nc[3]);
 int occ_distance_launches(const int nc[3], size_t tmp_bytes);
 inline size_t occupancy_bytes(long long ncells) { return (size_t)((ncells + 31) / 32) * 4; }
+
+// The memory of the last volume of a context that was destroyed, up to
+// VRC_VOLUME_KEEP bytes, for the next one of about its size. Volumes may be
+// destroyed by any thread, and after their context.
+struct KeptBlock {
+    std::mutex lock;
+    void* p = nullptr;
+    size_t bytes = 0;
+    bool closed = false;  // the context is gone
+    int device = 0;
+    // the block if it holds `need` bytes and not over twice as many
+    void* take(size_t need, size_t* got);
+    // keeps a block that no kernel uses any more, or frees it
+    void put(void* block, size_t n);
+    // frees what is kept; false if there was nothing
+    bool give_back(bool close);
+};
+// Device memory, giving the kept block back where there is none left.
+cudaError_t device_alloc(KeptBlock& kept, void** p, size_t bytes);
 
 // Process-unique id of a volume, TF or pre-integration table: identifies
 // the derived data cached for it even when an address is reused later.
@@ -245,6 +275,11 @@ struct vrc_context {
     uint8_t* d_dist = nullptr;       // occ_dist of the skip cells, and the passes' scratch
     uint8_t* d_dist_tmp = nullptr;
     size_t dist_bytes = 0, dist_tmp_bytes = 0;
+    void* d_stage = nullptr;         // slices of a volume on their way in, up to VRC_STAGE_KEEP bytes
+    size_t stage_bytes = 0;
+    std::shared_ptr<vrc::KeptBlock> kept = std::make_shared<vrc::KeptBlock>();
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr};
     int* d_prefix = nullptr;
     size_t prefix_bytes = 0;
     void* d_queue = nullptr;  // unfinished rays between the march's two kernels (march_queue_bytes)
@@ -304,6 +339,9 @@ struct vrc_volume {
     vrc::BrickLayout lod_L{};
     int lod_level = 0;                 // level d_lod holds: 1 = half resolution, k = 2^-k
     bool lod_on = false;
+    std::shared_ptr<vrc::KeptBlock> kept;  // the context's
+    void* d_block = nullptr;  // the allocation of the brick pool (device placement) and all min/max tables
+    size_t block_bytes = 0;
     float* d_bmin = nullptr;
     float* d_bmax = nullptr;
     vrc_cell_level levels[4];  // skip cells of edge 2, 4, 8 and 16 (when smaller than the brick; 2 up to 2^30 cells)
@@ -315,6 +353,21 @@ struct vrc_volume {
 // 8-Gvoxel volume, 8.6 GB of min/max tables).
 #ifndef VRC_CELL2_LOG2_MAX
 #define VRC_CELL2_LOG2_MAX 30
+#endif
+
+// Staged slices that a context keeps for its next upload, and the bytes of a
+// slab (at least a layer of bricks).
+#ifndef VRC_STAGE_KEEP
+#define VRC_STAGE_KEEP (128u << 20)
+#endif
+#ifndef VRC_SLAB_BYTES
+#define VRC_SLAB_BYTES (56u << 20)
+#endif
+// The largest block of a destroyed volume that a context keeps: cudaMalloc and
+// cudaFree of 512^3 u16's 505 MB took 640 us a new time step of 2990. Given back to the next volume, on
+// the first allocation that finds no memory, and with the context.
+#ifndef VRC_VOLUME_KEEP
+#define VRC_VOLUME_KEEP (1u << 30)
 #endif
 
 namespace vrc {
