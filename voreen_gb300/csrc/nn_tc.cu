@@ -19,7 +19,11 @@
 // per tile rather than three times. Warp roles: 0 = TMA producer, 1 = MMA
 // issuer and tensor-memory owner, 2..5 = epilogue (tensor memory -> bias,
 // activation -> global). Two sets of R accumulators let the epilogue of one
-// tile overlap the MMAs of the next. Every wait is bounded by %globaltimer:
+// tile overlap the MMAs of the next, and an output row is handed over when its
+// own MMAs are done: a CTA has one to three tiles, so the last one's epilogue
+// is in sight (handed over a tile at a time, the five layers of a 960x540
+// frame's upsampler took 10 us more of 121; 64 -> 64 at 480x270 runs the tensor
+// pipe 35 % of the time, at 70 cycles an MMA of N = 64). Every wait is bounded by %globaltimer:
 // the pipeline waits by a host-settable limit (vrc_nn_set_wait_limit, 200 ms
 // by default); on a timeout the CTA records an error code, waits for its own
 // copies and MMAs in flight (bounded by a fixed 200 ms, whatever the pipeline
@@ -45,7 +49,7 @@ constexpr int EPI_WARPS = 4;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr unsigned long long WAIT_NS = 200ull * 1000ull * 1000ull;
 constexpr float LEAK = 0.05f;
-constexpr int NBARS = 2 * MAX_STAGES + 2 + 2 + 2;  // full, empty, tmem full, tmem empty, weights, mma done
+constexpr int NBARS = 2 * MAX_STAGES + 2 * MAX_ROWS + 2 + 2;  // full, empty, tmem full (a row each), tmem empty, weights, mma done
 constexpr size_t SMEM_BUDGET = 224 * 1024;  // of the 227 KB a CTA may hold
 
 struct TcParams {
@@ -199,8 +203,7 @@ __global__ void __launch_bounds__(THREADS, 1)
     float* s_bias = reinterpret_cast<float*>(s_tmem + 4);  // this CTA's n_tile biases
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t full0 = su32(bars), empty0 = su32(bars + MAX_STAGES), tfull0 = su32(bars + 2 * MAX_STAGES),
-                   tempty0 = su32(bars + 2 * MAX_STAGES + 2), wbar = su32(bars + 2 * MAX_STAGES + 4),
-                   dbar = su32(bars + 2 * MAX_STAGES + 5);
+                   tempty0 = su32(bars + 2 * MAX_STAGES + 2 * MAX_ROWS), wbar = tempty0 + 16, dbar = tempty0 + 24;
     const int split = blockIdx.x % p.n_split;
     const int cta = blockIdx.x / p.n_split, ncta = gridDim.x / p.n_split;
     const int S = p.stages;
@@ -211,7 +214,7 @@ __global__ void __launch_bounds__(THREADS, 1)
             mbar_init(empty0 + 8 * s, 1);
         }
         for (int a = 0; a < 2; ++a) {
-            mbar_init(tfull0 + 8 * a, 1);
+            for (int o = 0; o < R; ++o) mbar_init(tfull0 + 8 * (a * R + o), 1);
             mbar_init(tempty0 + 8 * a, EPI_WARPS * 32);
         }
         mbar_init(wbar, 1);
@@ -319,8 +322,8 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                     mma_commit(empty0 + 8 * s);  // the stage is free once these MMAs have read it
                 }
+                if (ok && r >= 2) mma_commit(tfull0 + 8 * (acc * R + r - 2));  // output row r - 2 is complete
             }
-            if (ok) mma_commit(tfull0 + 8 * acc);
         }
         // every MMA issued by this thread has completed before tensor memory is freed
         mma_commit(dbar);
@@ -333,14 +336,16 @@ __global__ void __launch_bounds__(THREADS, 1)
         int tl = 0;
         for (int t = cta; t < p.pix_tiles; t += ncta, ++tl) {
             const int acc = tl & 1;
-            if (!mbar_wait(tfull0 + 8 * acc, (tl >> 1) & 1, s_abort, p.wait_ns, 256)) {
-                record_error(p.err, s_abort, 5);
-                break;
-            }
-            tc_fence_after();
             const TileCoord tc = tile_coord(p, t);
             const int x = tc.x0 + i;
+            bool ok = true;
             for (int o = 0; o < R; ++o) {
+                if (!mbar_wait(tfull0 + 8 * (acc * R + o), (tl >> 1) & 1, s_abort, p.wait_ns, 64)) {
+                    record_error(p.err, s_abort, 5);
+                    ok = false;
+                    break;
+                }
+                tc_fence_after();
                 const int y = tc.y0 + o;
                 for (int j0 = 0; j0 < p.n_tile; j0 += 16) {
                     uint32_t r[16];
@@ -370,6 +375,7 @@ __global__ void __launch_bounds__(THREADS, 1)
                     }
                 }
             }
+            if (!ok) break;
             tc_fence_before();
             mbar_arrive(tempty0 + 8 * acc);
         }
