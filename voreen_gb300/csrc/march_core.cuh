@@ -32,8 +32,9 @@
 //    is two FMAs an axis on per-ray constants. Together, us per frame before
 //    and after (bits unchanged): 512^3 u16 shaded DVR at 1080p 678 -> 475, its
 //    MIP 830 -> 661, pre-integrated 854 -> 605, 2048x2048x1024 tubes at 4K
-//    21,600 -> 15,440, 64 mixed requests 15,090 -> 11,030; with the lanes a
-//    ray, shaded DVR 475 -> 389, 64^3 u8 at 256^2 111 -> 54;
+//    21,600 -> 15,430, 64 mixed requests 15,100 -> 11,030; then the lanes a
+//    ray and the queue, shaded DVR 475 -> 388, pre-integrated 605 -> 487,
+//    64^3 u8 at 256^2 81 -> 48;
 //  * gradients (central differences, mod_gradients.frag:202-214) are six
 //    lookups at +-1/dim in texture space, clamped like the intensity sample
 //    and read from the centre's brick apron (another brick only when rounding
@@ -1583,6 +1584,7 @@ cudaError_t launch_group(const MarchParams& p, int num_sms, cudaStream_t s) {
 // full. The queue: one lane a ray, and the rays unfinished when the tiles run
 // out go on with 8 lanes each (half of a tube frame's gain with 4); it costs
 // the marching loop 3 % of its rate, which 4K frames do not get back.
+// Pre-integrated frames follow the same lines (1080p 605 -> 487).
 // MIP, MOP and MIDA go on to the end of the volume, so their rays are long
 // everywhere and the queue only adds to the work (512^3 MIP at 1080p 655 ->
 // 782 us, 1280x720 628 -> 970); they take 4 lanes up to 16,200 tiles (MIP 611

@@ -37,11 +37,12 @@ LAYERS = [  # name, Cin, Cout, activation (2: leaky ReLU, 0: none)
 LEAK = 0.05
 # Inference layers run on the tcgen05 convolution where it is faster than the
 # mma.sync one on a GB300 at 960 x 540 (measured per layer, microseconds,
-# tcgen05 / mma.sync): enc2a 23 / 25, enc2b 33 / 41, bota 15 / 29, botb 31 / 50,
-# dec2b 33 / 41. With 32 or fewer output channels an MMA of N <= 32 costs
+# tcgen05 / mma.sync): enc2a 19 / 25, enc2b 27 / 37, bota 14 / 31, botb 25 / 51,
+# dec2b 27 / 37. With 32 or fewer output channels an MMA of N <= 32 costs
 # about as much as one of N = 64, so the full-resolution layers (enc1a/b,
-# dec1b, head: 40-54 / 25-39) and the decoder inputs [upsample | skip]
-# (fused on load by the mma.sync form) stay on mma.sync.
+# dec1b, head: 41-55 / 23-37) and the decoder inputs [upsample | skip]
+# (fused on load by the mma.sync form: 92 / 93, tcgen05 113 / 137 after an
+# upsampling pass) stay on mma.sync.
 TC_LAYERS = ("enc2a", "enc2b", "bota", "botb", "dec2b")
 # Output-channel slices per CTA of the tcgen05 convolution, chosen so each
 # slice's weights (9 x Cin x Cout / split BF16) stay in shared memory beside
