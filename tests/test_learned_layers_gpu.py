@@ -85,3 +85,41 @@ def test_wide_pool_and_head_equal_the_scalar_forms(vrc_lib, n, h, w):
         out = buf[shift:shift + ref.numel()].reshape(ref.shape).double()
         # a few FP32 roundings of values up to |feature| + 1
         assert ((out - ref).abs() <= 8 * 2.0 ** -24 * (feat.abs().max().double() + 1)).all()
+
+
+@pytest.mark.parametrize("h,w", [(16, 16), (70, 130), (200, 312)])
+def test_chained_launches_see_what_came_before(vrc_lib, h, w):
+    """Layers that read what the launch before wrote, into buffers that the
+    launch before that read, with weights that another kernel just changed:
+    the same bits as with a synchronisation after every call."""
+    import torch
+    L, c = v.lib(), 64
+    seen = []
+    for wait in (True, False):
+        g = torch.Generator(device="cuda").manual_seed(h + w)
+        a = torch.randn((1, h, w, c), device="cuda", generator=g).to(torch.bfloat16)
+        b, pooled = torch.zeros_like(a), torch.zeros((1, h // 2, w // 2, c), dtype=torch.bfloat16, device="cuda")
+        w0 = (torch.randn((c, 3, 3, c), device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+        wt, wtc, bias = w0.clone(), torch.empty_like(w0), torch.randn(c, device="cuda", generator=g) * 0.1
+        sums, err = [], torch.zeros(1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+
+        def call(r):
+            assert r == 0
+            if wait:
+                torch.cuda.synchronize()
+
+        for i in range(12):
+            wt.copy_(torch.roll(w0, i, 0))
+            call(L.vrc_nn_weights_tc(_p(wt), c, c, 0, 1, _p(wtc), None))
+            call(L.vrc_nn_conv3x3_fwd(_p(a), 1, h, w, c, _p(wt), _p(bias), c, 2, _p(b), 0, None))
+            call(L.vrc_nn_conv3x3_tc(_p(b), c, None, 0, 1, h, w, _p(wtc), _p(bias), c, 1, 2, _p(a), 0, _p(err), None))
+            call(L.vrc_nn_avgpool2(_p(a), 1, h, w, c, C.c_float(1.0), _p(pooled), None))
+            call(L.vrc_nn_conv3x3_tc(_p(a), c, None, 0, 1, h, w, _p(wtc), _p(bias), c, 1, 2, _p(b), 0, _p(err), None))
+            call(L.vrc_nn_conv3x3_fwd(_p(b), 1, h, w, c, _p(wt), _p(bias), c, 2, _p(a), 0, None))
+            sums += [pooled.clone(), b.clone(), a.clone()]
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        seen.append(sums)
+    assert all(torch.equal(x, y) for x, y in zip(*seen))
+    assert all(bool(torch.isfinite(x.float()).all()) and float(x.float().abs().sum()) > 0 for x in seen[0])

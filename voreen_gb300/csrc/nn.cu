@@ -14,6 +14,7 @@
 #include <algorithm>
 
 #include "../../include/vrc_nn.h"
+#include "nn_launch.cuh"
 
 namespace {
 
@@ -93,9 +94,8 @@ template <int COUT, int RPW> struct FwdTile {
 // Ca + Cb and `in` is A. With in_b == nullptr the input is `in` as is.
 template <int COUT, int RPW>
 __global__ void __launch_bounds__(256, COUT <= 32 ? 3 : (COUT == 64 ? 2 : 1))
-    conv3x3_fwd_kernel(const __nv_bfloat16* __restrict__ in, int N, int H, int W, int Cin,
-                       const __nv_bfloat16* __restrict__ wt, const float* __restrict__ bias, int relu, void* out,
-                       int out_f32, const __nv_bfloat16* __restrict__ in_b, int Ca) {
+    conv3x3_fwd_kernel(const __nv_bfloat16* in, int N, int H, int W, int Cin, const __nv_bfloat16* wt, const float* bias,
+                       int relu, void* out, int out_f32, const __nv_bfloat16* in_b, int Ca) {
     using FT = FwdTile<COUT, RPW>;
     constexpr int NT = COUT / 8;
     extern __shared__ __align__(16) __nv_bfloat16 smem[];  // [2] x { [TH+2][18][PIX_PAD], [9][COUT][PIX_PAD] }
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(256, COUT <= 32 ? 3 : (COUT == 64 ? 2 : 1))
         }
         cp_async_commit();
     };
+    after_previous();
     stage(0, 0);
     for (int c0 = 0, set = 0; c0 < Cin; c0 += 16, set ^= 1) {
         if (c0 + 16 < Cin) {
@@ -197,6 +198,12 @@ __global__ void __launch_bounds__(256, COUT <= 32 ? 3 : (COUT == 64 ? 2 : 1))
     }
     // epilogue: bias, optional ReLU, store (d0,d1: pixel g; d2,d3: pixel g + 8)
     const int g = lane >> 2, t = lane & 3;
+    float bias0[NT], bias1[NT];  // before the stores, which the loads may not pass
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        bias0[j] = bias ? bias[j * 8 + 2 * t] : 0.f;
+        bias1[j] = bias ? bias[j * 8 + 2 * t + 1] : 0.f;
+    }
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
         const int y = y0 + warp * RPW + r;
@@ -204,12 +211,11 @@ __global__ void __launch_bounds__(256, COUT <= 32 ? 3 : (COUT == 64 ? 2 : 1))
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
             const int co = j * 8 + 2 * t;
-            const float b0 = bias ? bias[co] : 0.f, b1 = bias ? bias[co + 1] : 0.f;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 const int x = x0 + g + 8 * h;
                 if (x >= W) continue;
-                float v0 = acc[r][j][2 * h] + b0, v1 = acc[r][j][2 * h + 1] + b1;
+                float v0 = acc[r][j][2 * h] + bias0[j], v1 = acc[r][j][2 * h + 1] + bias1[j];
                 if (relu == 1) {
                     v0 = fmaxf(v0, 0.f);
                     v1 = fmaxf(v1, 0.f);
@@ -239,8 +245,7 @@ cudaError_t conv_fwd_t(const __nv_bfloat16* in, int N, int H, int W, int Cin, co
     if (e != cudaSuccess) return e;
     dim3 grid((W + 15) / 16, (H + FT::TH - 1) / FT::TH, N);
     // one chunk needs one set of stages
-    k<<<grid, 256, (Cin > 16 ? 2 : 1) * FT::BYTES, s>>>(in, N, H, W, Cin, w, bias, relu, out, out_f32, in_b, Ca);
-    return cudaGetLastError();
+    return launch_chained(k, grid, 256, (Cin > 16 ? 2 : 1) * FT::BYTES, s, in, N, H, W, Cin, w, bias, relu, out, out_f32, in_b, Ca);
 }
 
 // ---------------------------------------------------------------------------
@@ -269,8 +274,8 @@ template <int COUT> struct WgradTile {
 
 template <int COUT>
 __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
-    conv3x3_wgrad_kernel(const __nv_bfloat16* __restrict__ in, const __nv_bfloat16* __restrict__ dout, int N, int H,
-                         int W, int Cin, float* dw, float* dbias, int tiles_per_cta) {
+    conv3x3_wgrad_kernel(const __nv_bfloat16* in, const __nv_bfloat16* dout, int N, int H, int W, int Cin, float* dw,
+                         float* dbias, int tiles_per_cta) {
     using WT = WgradTile<COUT>;
     constexpr int MT = COUT / 16;               // m16 tiles along COUT
     constexpr int NG = 8 / MT;                  // warps sharing one m tile, each owns 8/NG n-tiles
@@ -309,6 +314,7 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
         cp_async_commit();
     };
     const int t_begin = blockIdx.x * tiles_per_cta, t_end = min(ntiles, t_begin + tiles_per_cta);
+    after_previous();
     if (t_begin < t_end) stage(t_begin, 0);
     for (int tile = t_begin, set = 0; tile < t_end; ++tile, set ^= 1) {
         if (tile + 1 < t_end) {
@@ -382,8 +388,7 @@ cudaError_t conv_wgrad_t(const __nv_bfloat16* in, const __nv_bfloat16* dout, int
     const int runs = (WGRAD_CTAS + blocks - 1) / blocks;
     const int per = max(1, min(32, (ntiles + runs - 1) / runs));
     dim3 grid((ntiles + per - 1) / per, 3, (Cin + WG_CI - 1) / WG_CI);
-    k<<<grid, 256, WT::BYTES, s>>>(in, dout, N, H, W, Cin, dw, dbias, per);
-    return cudaGetLastError();
+    return launch_chained(k, grid, 256, WT::BYTES, s, in, dout, N, H, W, Cin, dw, dbias, per);
 }
 
 // ---------------------------------------------------------------------------
@@ -405,12 +410,12 @@ __device__ __forceinline__ float pool4(__nv_bfloat16 a, __nv_bfloat16 b, __nv_bf
     return 0.25f * scale * s;
 }
 template <int V>
-__global__ void avgpool_kernel(const __nv_bfloat16* __restrict__ in, int rows, int H, int W, int C, float scale,
-                               __nv_bfloat16* __restrict__ out) {
+__global__ void avgpool_kernel(const __nv_bfloat16* in, int rows, int H, int W, int C, float scale, __nv_bfloat16* out) {
     struct alignas(2 * V) Vec {
         __nv_bfloat16 v[V];
     };
     const int Ho = H / 2, Wo = W / 2, CV = C / V;
+    after_previous();
     for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
         const int b = row / Ho, y = row - b * Ho;
         const Vec* p = reinterpret_cast<const Vec*>(in + ((size_t)b * H + 2 * y) * W * C);
@@ -479,26 +484,26 @@ __device__ __forceinline__ float bilerp_base(const float* base, int b, int H, in
 // 16-byte load each. HBM is the bound (64 + 16 bytes a low-resolution pixel
 // read, 64 written). A channel a thread, with 64-bit divisions and scalar
 // loads, took 57.7 us at 960x540, this 16.6.
-__device__ __forceinline__ float4 bilerp_base4(const float4* __restrict__ p, int H, int W, int oy, int ox) {
+__device__ __forceinline__ float4 bilerp_base4(const float4* p, int H, int W, int oy, int ox) {
     const float sy = fmaxf((oy + 0.5f) * 0.5f - 0.5f, 0.f), sx = fmaxf((ox + 0.5f) * 0.5f - 0.5f, 0.f);
     const int y0 = min((int)sy, H - 1), x0 = min((int)sx, W - 1);
     const int y1 = min(y0 + 1, H - 1), x1 = min(x0 + 1, W - 1);
     const float fy = sy - y0, fx = sx - x0;
-    const float4 a = __ldg(p + (size_t)y0 * W + x0), b = __ldg(p + (size_t)y0 * W + x1);
-    const float4 c = __ldg(p + (size_t)y1 * W + x0), d = __ldg(p + (size_t)y1 * W + x1);
+    const float4 a = p[(size_t)y0 * W + x0], b = p[(size_t)y0 * W + x1];
+    const float4 c = p[(size_t)y1 * W + x0], d = p[(size_t)y1 * W + x1];
     auto mix = [&](float v00, float v01, float v10, float v11) {
         return (v00 * (1.f - fx) + v01 * fx) * (1.f - fy) + (v10 * (1.f - fx) + v11 * fx) * fy;
     };
     return make_float4(mix(a.x, b.x, c.x, d.x), mix(a.y, b.y, c.y, d.y), mix(a.z, b.z, c.z, d.z), mix(a.w, b.w, c.w, d.w));
 }
-__global__ void __launch_bounds__(128) head_fwd_kernel(const float4* __restrict__ feat4, const float4* __restrict__ base,
-                                                       int rows, int H, int W, float4* __restrict__ out) {
+__global__ void __launch_bounds__(128) head_fwd_kernel(const float4* feat4, const float4* base, int rows, int H, int W, float4* out) {
     const int Ho = 2 * H, Wo = 2 * W;
+    after_previous();
     for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
         const int b = row / Ho, oy = row - b * Ho;
         const float4* f4 = feat4 + ((size_t)b * H + oy / 2) * W * 4 + 2 * (oy & 1);
         for (int ox = blockIdx.x * 128 + threadIdx.x; ox < Wo; ox += gridDim.x * 128) {
-            const float4 f = __ldg(f4 + (size_t)(ox >> 1) * 4 + (ox & 1));
+            const float4 f = f4[(size_t)(ox >> 1) * 4 + (ox & 1)];
             const float4 u = bilerp_base4(base + (size_t)b * H * W, H, W, oy, ox);
             out[(size_t)row * Wo + ox] = make_float4(f.x + u.x, f.y + u.y, f.z + u.z, f.w + u.w);
         }
@@ -786,10 +791,8 @@ int vrc_nn_avgpool2(const void* in, int N, int H, int W, int C, float scale, voi
     const auto* i = static_cast<const __nv_bfloat16*>(in);
     auto* o = static_cast<__nv_bfloat16*>(out);
     if (wide)
-        avgpool_kernel<8><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(i, rows, H, W, C, scale, o);
-    else
-        avgpool_kernel<1><<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(i, rows, H, W, C, scale, o);
-    return status_of(cudaGetLastError());
+        return status_of(launch_chained(avgpool_kernel<8>, grid, 256, 0, static_cast<cudaStream_t>(stream), i, rows, H, W, C, scale, o));
+    return status_of(launch_chained(avgpool_kernel<1>, grid, 256, 0, static_cast<cudaStream_t>(stream), i, rows, H, W, C, scale, o));
 }
 
 int vrc_nn_upsample2(const void* in, int N, int H, int W, int C, float scale, void* out, void* stream) {
@@ -818,8 +821,8 @@ int vrc_nn_head_fwd(const float* feat16, const float* base, int N, int H, int W,
         head_fwd_unaligned_kernel<<<ew_grid((long long)N * H * W * 16), 256, 0, st>>>(feat16, base, N, H, W, out);
     } else {
         const dim3 grid((unsigned)std::max(1, (2 * W + 127) / 128), (unsigned)std::max(1, std::min(rows, 65535)));
-        head_fwd_kernel<<<grid, 128, 0, st>>>(reinterpret_cast<const float4*>(feat16), reinterpret_cast<const float4*>(base),
-                                              rows, H, W, reinterpret_cast<float4*>(out));
+        return status_of(launch_chained(head_fwd_kernel, grid, 128, 0, st, reinterpret_cast<const float4*>(feat16),
+                                        reinterpret_cast<const float4*>(base), rows, H, W, reinterpret_cast<float4*>(out)));
     }
     return status_of(cudaGetLastError());
 }

@@ -38,6 +38,7 @@
 #include <mutex>
 
 #include "../../include/vrc_nn.h"
+#include "nn_launch.cuh"
 
 namespace {
 
@@ -222,6 +223,7 @@ __global__ void __launch_bounds__(THREADS, 1)
         *s_abort = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    after_previous();  // also before tensor memory, which a CTA of the layer before may hold
     for (int j = threadIdx.x; j < p.n_tile; j += THREADS) s_bias[j] = p.bias ? p.bias[split * p.n_tile + j] : 0.f;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(s_tmem)),
@@ -562,8 +564,7 @@ int vrc_nn_conv3x3_tc(const void* in0, int C0, const void* in1, int C1, int N, i
     long long per_split = sms / n_split;
     if (per_split < 1) per_split = 1;
     if (per_split > pix_tiles) per_split = pix_tiles;
-    k<<<(unsigned)(per_split * n_split), THREADS, smem, static_cast<cudaStream_t>(stream)>>>(m0, m1, p);
-    return status(cudaGetLastError());
+    return status(launch_chained(k, dim3((unsigned)(per_split * n_split)), THREADS, smem, static_cast<cudaStream_t>(stream), m0, m1, p));
 }
 
 }  // extern "C"
