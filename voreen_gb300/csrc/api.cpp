@@ -283,7 +283,7 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_dist_tmp);
     cudaFree(c->d_stage);
     c->kept->give_back(true);
-    for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1]})
+    for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1], c->queued})
         if (ev) cudaEventDestroy(ev);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     cudaFree(c->d_prefix);
@@ -441,11 +441,13 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             stage = (char*)staging;
         }
         if (e != cudaSuccess) return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: staging allocation failed");
-        if (!ctx->copy_stream) {
-            e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
-            for (cudaEvent_t* ev : {&ctx->copied[0], &ctx->copied[1], &ctx->consumed[0], &ctx->consumed[1]})
-                if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
-        }
+        if (!ctx->copy_stream) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
+        for (cudaEvent_t* ev : {&ctx->copied[0], &ctx->copied[1], &ctx->consumed[0], &ctx->consumed[1], &ctx->queued})
+            if (e == cudaSuccess && !*ev) e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming);
+        // the copies come after what the caller has queued on the context's
+        // stream, which may still be writing pinned voxels
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->queued, ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->copy_stream, ctx->queued, 0);
         int have = 0;  // slices copied
         for (int l0 = 0, k = 0; l0 < L.nb[2] && e == cudaSuccess; l0 += layers, k ^= 1) {
             const int l1 = std::min(l0 + layers, L.nb[2]);

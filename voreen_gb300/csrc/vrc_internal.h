@@ -279,7 +279,7 @@ struct vrc_context {
     size_t stage_bytes = 0;
     std::shared_ptr<vrc::KeptBlock> kept = std::make_shared<vrc::KeptBlock>();
     cudaStream_t copy_stream = nullptr;
-    cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr};
+    cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr}, queued = nullptr;
     int* d_prefix = nullptr;
     size_t prefix_bytes = 0;
     void* d_queue = nullptr;  // unfinished rays between the march's two kernels (march_queue_bytes)
