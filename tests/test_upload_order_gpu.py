@@ -1,5 +1,8 @@
-"""Host voxels are copied on a stream of their own: their place among the work of
-the context, which is ordered on the context's stream."""
+"""Host voxels are copied on a stream of their own, through memory that the context
+keeps: their place among the work of the context, which is ordered on the
+context's stream, and uploads of several threads."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -39,3 +42,27 @@ def test_upload_waits_for_the_context_stream(ctx, dims):
         vol.close()
         np.testing.assert_array_equal(lo, want[0])
         np.testing.assert_array_equal(hi, want[1])
+
+
+def test_uploads_of_two_threads_share_a_context(ctx):
+    """Each thread's volumes hold its own voxels (three slabs each; the calls
+    release the interpreter lock)."""
+    voxels = [np.random.default_rng(k).integers(0, 256, (150, 1024, 1024), dtype=np.uint8) for k in range(2)]
+    want = [_brick_minmax(vox) for vox in voxels]
+    wrong, start = [], threading.Barrier(2)
+
+    def upload(k):
+        start.wait(60)
+        for _ in range(6):
+            vol = v.Volume(ctx, voxels[k])
+            lo, hi, _ = vol.brick_minmax()
+            vol.close()
+            if not (np.array_equal(lo, want[k][0]) and np.array_equal(hi, want[k][1])):
+                wrong.append(k)
+
+    threads = [threading.Thread(target=upload, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong

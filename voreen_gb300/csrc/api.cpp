@@ -341,6 +341,9 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         delete v;
         return fail(ctx, VRC_ERR_UNSUPPORTED, "vrc_volume_upload: more than 2^31 bricks");
     }
+    // the ring, the copy stream and its events are the context's: one upload at
+    // a time has them, until both streams are done with it
+    std::unique_lock<std::mutex> staged(ctx->stage_lock, std::defer_lock);
     void* staging = nullptr;  // a ring of slices too large to keep
     const void* registered = nullptr;  // caller's host voxels registered for direct device reads
     cudaError_t e = cudaSuccess;
@@ -432,6 +435,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         const int Z = desc->dims[2];
         const int layers = (int)std::min<size_t>(std::max<size_t>(VRC_SLAB_BYTES / (slice * L.B), 1), L.nb[2]);
         const int ring = (int)std::min<long long>(2ll * layers * L.B + vrc::APRON_LO + vrc::APRON_HI, Z);
+        staged.lock();
         char* stage = nullptr;
         if (ring * slice <= VRC_STAGE_KEEP) {
             e = ensure(ctx, &ctx->d_stage, &ctx->stage_bytes, ring * slice);

@@ -277,6 +277,7 @@ struct vrc_context {
     size_t dist_bytes = 0, dist_tmp_bytes = 0;
     void* d_stage = nullptr;         // slices of a volume on their way in, up to VRC_STAGE_KEEP bytes
     size_t stage_bytes = 0;
+    std::mutex stage_lock;           // the upload that has them and the copy stream
     std::shared_ptr<vrc::KeptBlock> kept = std::make_shared<vrc::KeptBlock>();
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr}, queued = nullptr;
