@@ -307,8 +307,8 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
         }
         for (int i = tid; i < 8 * 18 * (WG_CI / 8); i += 256) {
             const int p = i / (WG_CI / 8), v8 = i % (WG_CI / 8);
-            const int gy = y0 + p / 18 + kh - 1, gx = x0 + p % 18 - 1;
-            const bool ok = gy >= 0 && gy < H && gx >= 0 && gx < W && ci0 + v8 * 8 < Cin;
+            const int y = y0 + p / 18, gy = y + kh - 1, gx = x0 + p % 18 - 1;
+            const bool ok = y < H && gy >= 0 && gy < H && gx >= 0 && gx < W && ci0 + v8 * 8 < Cin;
             cp_async16(si + (p * WT::IS + v8 * 8) * 2, ok ? in + (((size_t)n * H + gy) * W + gx) * Cin + ci0 + v8 * 8 : in, ok);
         }
         cp_async_commit();
@@ -325,6 +325,14 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
         }
         __syncthreads();
         const __nv_bfloat16 *s_d = smem + set * WT::STAGE, *s_i = s_d + WT::D;
+        // Where the tile overhangs the image on the right, the image's last
+        // column is staged for kw = 1 and 2, but its output pixel at kw = 0
+        // lies outside: out of that operand (pixels 2t, 2t + 1 and + 8 in this
+        // thread's registers), as 0 times an infinity would not be 0. Rows and
+        // the columns beyond it are zeros already.
+        const int over = W - (tile % tiles_x) * 16 - 2 * (lane & 3);
+        const uint32_t keep0 = over == 0 ? 0xffff0000u : over == 1 ? 0x0000ffffu : ~0u;
+        const uint32_t keep8 = over == 8 ? 0xffff0000u : over == 9 ? 0x0000ffffu : ~0u;
         if (sums_bias)
             for (int p = tid / COUT; p < 128; p += PARTS) bsum += __bfloat162float(s_d[p * WT::DS + tid % COUT]);
 #pragma unroll
@@ -345,6 +353,7 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
                     const int p = row * 18 + kw + ((lane >> 3) & 1) * 8 + (lane & 7);
                     uint32_t b0, b1, b2, b3;
                     ldsm_x4_t(smem_u32(s_i + p * WT::IS + nt * 8), b0, b1, b2, b3);
+                    if (kw == 0) b0 &= keep0, b1 &= keep8, b2 &= keep0, b3 &= keep8;
                     mma_bf16(acc[kw][j], a0, a1, a2, a3, b0, b1);
                     if (j + 1 < NTW) mma_bf16(acc[kw][j + 1], a0, a1, a2, a3, b2, b3);
                 }
