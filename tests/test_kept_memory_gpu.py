@@ -1,0 +1,119 @@
+"""The device memory that a context keeps for its next volume: who may free a
+volume and when, and who gets the memory back."""
+import gc
+import threading
+
+import numpy as np
+import pytest
+
+import voreen_gb300 as v
+from voreen_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+MIB = 1 << 20
+
+
+def _free():
+    import torch
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def _voxels(n, seed):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    vox = torch.randint(0, 256, (n, n, n), dtype=torch.uint8, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    return vox
+
+
+def _volume(ctx, n=256, seed=1):
+    return v.Volume(ctx, _voxels(n, seed))
+
+
+def _frame(ctx, vol, out=None):
+    p = v.default_params(128, 96)
+    pos, focus, near, far = synth.orbit_camera(vol.dims, (1.0, 1.0, 1.0), 30.0, 20.0, 1.1)
+    p.camera, p.entry_exit_mode = v.make_camera(pos, focus, near=near, far=far), v.EE_ANALYTIC
+    tf = v.TransferFunction(ctx, v.TransferFunction.bake([(0.0, (0, 0, 0, 0)), (1.0, (255, 200, 100, 60))], 256), (0.0, 1.0))
+    image, _ = v.render(ctx, vol, tf, p, out_format=v.OUT_RGBA32F)
+    tf.close()
+    return np.array(image)
+
+
+def test_volume_destroyed_while_another_stream_captures(vrc_lib):
+    """A thread frees volumes while another one captures a graph (thread-local
+    mode): the capture is not touched, the memory serves the next volume."""
+    import torch
+    ctx = v.Context(0)
+    want = _frame(ctx, _volume(ctx, seed=2))
+    vol = _volume(ctx)
+    _frame(ctx, vol)
+    a = torch.zeros(1024, device="cuda")
+    torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        graph.capture_begin(capture_error_mode="thread_local")
+        a.add_(1.0)
+        t = threading.Thread(target=vol.close)
+        t.start()
+        t.join()
+        a.add_(1.0)
+        graph.capture_end()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((a == 2.0).all())
+    np.testing.assert_array_equal(_frame(ctx, _volume(ctx, seed=2)), want)
+    ctx.close()
+
+
+def test_volume_destroyed_under_a_frame_on_another_stream(vrc_lib):
+    """A frame that vrc_render_noalloc has queued on the caller's stream, behind
+    other work, shows the volume it was given, though that was destroyed and
+    the next one uploaded meanwhile."""
+    import torch
+    ctx = v.Context(0)
+    p = v.default_params(128, 96)
+    tf = v.TransferFunction(ctx, v.TransferFunction.bake([(0.0, (0, 0, 0, 0)), (1.0, (255, 200, 100, 60))], 256), (0.0, 1.0))
+    busy, side = torch.ones(1 << 28, device="cuda"), torch.cuda.Stream()
+    seen, first, second = [], _voxels(256, 1), _voxels(256, 3)
+    for hurry in (False, True):
+        vol = v.Volume(ctx, first)
+        pos, focus, near, far = synth.orbit_camera(vol.dims, (1.0, 1.0, 1.0), 30.0, 20.0, 1.1)
+        p.camera, p.entry_exit_mode = v.make_camera(pos, focus, near=near, far=far), v.EE_ANALYTIC
+        out = torch.zeros((96, 128, 4), device="cuda")
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            for _ in range(60):  # some 20 ms
+                busy.mul_(1.0)
+        v.render_noalloc(vol, tf, p, None, None, out, v.OUT_RGBA32F, side.cuda_stream)
+        if not hurry:
+            torch.cuda.synchronize()
+        vol.close()
+        other = v.Volume(ctx, second)
+        torch.cuda.synchronize()
+        seen.append(out.cpu().numpy())
+        other.close()
+    assert seen[0].any()
+    np.testing.assert_array_equal(seen[0], seen[1])
+    tf.close()
+    ctx.close()
+
+
+def test_memory_returns_with_the_context_whoever_goes_first(vrc_lib):
+    """A context closed before its volumes, and one after: nothing stays."""
+    import torch
+    c = v.Context(0)
+    _frame(c, _volume(c, 64))
+    c.close()
+    gc.collect()
+    torch.cuda.empty_cache()
+    before = _free()
+    for context_first in (True, False):
+        ctx = v.Context(0)
+        vol, host = _volume(ctx, 512), v.Volume(ctx, np.ones((200, 512, 512), np.uint8))
+        _frame(ctx, vol)
+        for x in (ctx, vol, host) if context_first else (vol, host, ctx):
+            x.close()
+        torch.cuda.empty_cache()
+        assert _free() >= before - 4 * MIB, context_first

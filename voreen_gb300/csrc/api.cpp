@@ -509,8 +509,11 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
 vrc_status vrc_volume_destroy(vrc_volume* v) {
     if (!v) return VRC_ERR_INVALID_ARG;
     if (v->kept) cudaSetDevice(v->kept->device);
-    // no frame on any stream reads the volume any more, as after a cudaFree
-    if (v->d_block && v->kept && cudaDeviceSynchronize() == cudaSuccess)
+    // What read the block did so on the context's stream, where alone the next
+    // volume writes it. Frames on streams of the caller's (vrc_render_noalloc)
+    // are what cudaFree waits for. (Not a wait for the device here: it would
+    // end any capture that another thread has under way.)
+    if (v->d_block && v->kept && !v->off_stream.load())
         v->kept->put(v->d_block, v->block_bytes);
     else
         cudaFree(v->d_block);

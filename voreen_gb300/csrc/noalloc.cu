@@ -93,6 +93,7 @@ struct DeviceScope {
 
 vrc_status render_noalloc(const vrc_volume* vol, const vrc_tf* tf, const vrc_render_params* p, const float* d_entry,
                           const float* d_exit, void* d_out, int out_format, cudaStream_t s, int dev) {
+    vol->off_stream.store(true);
     unsigned char* scratch = static_cast<unsigned char*>(g_scratch_addr[dev]);
     vrc::MarchParams P;
     vrc_status st = vrc::fill_params(nullptr, vol, p, P);

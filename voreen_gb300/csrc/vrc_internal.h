@@ -239,7 +239,7 @@ struct KeptBlock {
     int device = 0;
     // the block if it holds `need` bytes and not over twice as many
     void* take(size_t need, size_t* got);
-    // keeps a block that no kernel uses any more, or frees it
+    // keeps a block that only work on the context's stream has used, or frees it
     void put(void* block, size_t n);
     // frees what is kept; false if there was nothing
     bool give_back(bool close);
@@ -343,6 +343,7 @@ struct vrc_volume {
     std::shared_ptr<vrc::KeptBlock> kept;  // the context's
     void* d_block = nullptr;  // the allocation of the brick pool (device placement) and all min/max tables
     size_t block_bytes = 0;
+    mutable std::atomic<bool> off_stream{false};  // a frame went to a stream of the caller's
     float* d_bmin = nullptr;
     float* d_bmax = nullptr;
     vrc_cell_level levels[4];  // skip cells of edge 2, 4, 8 and 16 (when smaller than the brick; 2 up to 2^30 cells)
