@@ -106,6 +106,12 @@ vrc_status vrc_context_create(int device, vrc_context** out);
  * first: they keep a pointer to it. */
 vrc_status vrc_context_destroy(vrc_context* ctx);
 vrc_status vrc_context_synchronize(vrc_context* ctx);
+/* Between calls a context keeps the device memory of the last volume destroyed,
+ * up to 1 GiB, for its next volume of about that size, and up to 128 MB of
+ * staging for host voxels. It gives them back when one of its own allocations
+ * finds no memory, when it is destroyed, and here: for callers whose other
+ * allocations on the device need the room. */
+vrc_status vrc_context_trim(vrc_context* ctx);
 /* The context's cudaStream_t, for callers that order their own work with it. */
 void* vrc_context_stream(vrc_context* ctx);
 const char* vrc_status_string(vrc_status s);
@@ -140,10 +146,7 @@ vrc_status vrc_volume_upload(vrc_context* ctx, const vrc_volume_desc* desc, cons
 typedef enum { VRC_PLACE_DEVICE = 0, VRC_PLACE_HOST = 1 } vrc_placement;
 vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* desc, const void* voxels,
                                     int voxels_on_device, int brick_size, int placement, vrc_volume** out);
-/* The context keeps the device memory of the last volume destroyed, up to
- * 1 GiB, for its next volume of about that size, and up to 128 MB of staging
- * for host voxels; it gives the former back when one of its own allocations
- * finds no memory, and both when it is destroyed. */
+/* Frees a volume, or keeps its device memory for the next (vrc_context_trim). */
 vrc_status vrc_volume_destroy(vrc_volume* vol);
 /* Min/max of the normalised intensity (getVoxelNormalized) over the volume. */
 vrc_status vrc_volume_minmax(vrc_volume* vol, float* min_norm, float* max_norm);

@@ -100,6 +100,47 @@ def test_volume_destroyed_under_a_frame_on_another_stream(vrc_lib):
     ctx.close()
 
 
+def test_failing_allocations_give_the_memory_back(vrc_lib, tmp_path):
+    """An allocation of the context that finds no memory: what the context keeps
+    goes back first (a file of 550 GB of voxels; the volume itself)."""
+    import torch
+    ctx = v.Context(0)
+    raw = tmp_path / "huge.raw"
+    raw.write_bytes(b"\0" * 64)
+    (tmp_path / "huge.vvd").write_text(
+        '<?xml version="1.0" ?><VoreenData version="1"><Volumes><Volume><RawData filename="huge.raw" format="uint8" x="8192" '
+        'y="8192" z="8192" /></Volume></Volumes></VoreenData>')
+    desc = v.make_desc(v.U8, (8192, 8192, 8192))
+    one = torch.zeros(64, dtype=torch.uint8, device="cuda")
+
+    def load():
+        v.Volume.load_vvd(ctx, str(tmp_path / "huge.vvd"))
+
+    def upload():
+        import ctypes as C
+        h = C.c_void_p()
+        st = v.lib().vrc_volume_upload(ctx.handle, C.byref(desc), C.c_void_p(one.data_ptr()), 1, 0, C.byref(h))
+        if st:
+            raise v.VrcError(st, "upload")
+
+    for call in (load, upload, ctx.trim):
+        vol, host = _volume(ctx, 512), v.Volume(ctx, np.ones((250, 512, 512), np.uint8))
+        torch.cuda.empty_cache()
+        for x in (host, vol):
+            x.close()
+        held = _free()
+        if call != ctx.trim:
+            with pytest.raises(v.VrcError, match="OUT_OF_MEMORY"):
+                call()
+        else:
+            call()
+        # the 512^3 volume's block (214 MB) and the staging of the other (66 MB)
+        assert _free() - held >= 260 * MIB, call
+    vol = _volume(ctx, 512)  # and no error is left for the next call's launches
+    vol.close()
+    ctx.close()
+
+
 def test_memory_returns_with_the_context_whoever_goes_first(vrc_lib):
     """A context closed before its volumes, and one after: nothing stays."""
     import torch

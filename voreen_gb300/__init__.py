@@ -82,6 +82,10 @@ class Context:
     def synchronize(self):
         _check(lib().vrc_context_synchronize(self.handle), self, "vrc_context_synchronize")
 
+    def trim(self):
+        """Give back the device memory the context keeps for later calls."""
+        _check(lib().vrc_context_trim(self.handle), self, "vrc_context_trim")
+
     def close(self):
         if self.handle:
             lib().vrc_context_destroy(self.handle)

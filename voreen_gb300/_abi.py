@@ -92,6 +92,7 @@ SIGNATURES = {
     "vrc_context_create": (C.c_int, [C.c_int, P(VP)]),
     "vrc_context_destroy": (C.c_int, [VP]),
     "vrc_context_synchronize": (C.c_int, [VP]),
+    "vrc_context_trim": (C.c_int, [VP]),
     "vrc_context_stream": (VP, [VP]),
     "vrc_volume_upload": (C.c_int, [VP, P(VolumeDesc), VP, C.c_int, C.c_int, P(VP)]),
     "vrc_volume_destroy": (C.c_int, [VP]),

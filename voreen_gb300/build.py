@@ -25,6 +25,7 @@ COMMON = ["-std=c++17", "-O3", "-lineinfo", "-Xcompiler", "-fPIC,-fopenmp,-ffp-c
 # remaining plain arithmetic on that path from being fused as well.
 SOURCES = [
     ("api.cpp", []),
+    ("kept.cpp", []),
     ("synth.cpp", []),
     ("volume.cu", []),
     ("march.cu", ["-fmad=false"]),

@@ -16,48 +16,6 @@
 using vrc::BrickLayout;
 using vrc::MarchParams;
 
-namespace vrc {
-
-void* KeptBlock::take(size_t need, size_t* got) {
-    std::lock_guard<std::mutex> g(lock);
-    if (!p || bytes < need || bytes / 2 > need) return nullptr;
-    void* block = p;
-    *got = bytes;
-    p = nullptr;
-    return block;
-}
-
-void KeptBlock::put(void* block, size_t n) {
-    if (n <= VRC_VOLUME_KEEP) {
-        std::lock_guard<std::mutex> g(lock);
-        if (!closed) {
-            std::swap(p, block);
-            bytes = n;
-        }
-    }
-    cudaFree(block);
-}
-
-bool KeptBlock::give_back(bool close) {
-    void* block = nullptr;
-    {
-        std::lock_guard<std::mutex> g(lock);
-        std::swap(p, block);
-        closed = closed || close;
-    }
-    cudaFree(block);
-    return block != nullptr;
-}
-
-cudaError_t device_alloc(KeptBlock& kept, void** p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaErrorMemoryAllocation || !kept.give_back(false)) return e;
-    cudaGetLastError();
-    return cudaMalloc(p, bytes);
-}
-
-}  // namespace vrc
-
 namespace {
 
 vrc_status fail(vrc_context* ctx, vrc_status s, const std::string& msg) {
@@ -248,6 +206,12 @@ vrc_status vrc_context_create(int device, vrc_context** out) {
     if (device < 0 || device >= n) return VRC_ERR_INVALID_ARG;
     vrc_context* c = new (std::nothrow) vrc_context();
     if (!c) return VRC_ERR_OUT_OF_MEMORY;
+    try {
+        c->kept = std::make_shared<vrc::KeptMemory>();
+    } catch (const std::bad_alloc&) {
+        delete c;
+        return VRC_ERR_OUT_OF_MEMORY;
+    }
     c->device = c->kept->device = device;
     if ((e = cudaSetDevice(device)) != cudaSuccess || (e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device)) != cudaSuccess) {
@@ -281,7 +245,6 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_occ_coarse);
     cudaFree(c->d_dist);
     cudaFree(c->d_dist_tmp);
-    cudaFree(c->d_stage);
     c->kept->give_back(true);
     for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1], c->queued})
         if (ev) cudaEventDestroy(ev);
@@ -297,6 +260,13 @@ vrc_status vrc_context_destroy(vrc_context* c) {
 vrc_status vrc_context_synchronize(vrc_context* c) {
     if (!c) return VRC_ERR_INVALID_ARG;
     VRC_CUDA(c, cudaStreamSynchronize(c->stream));
+    return VRC_OK;
+}
+
+vrc_status vrc_context_trim(vrc_context* c) {
+    if (!c) return VRC_ERR_INVALID_ARG;
+    VRC_CUDA(c, cudaSetDevice(c->device));
+    c->kept->give_back();
     return VRC_OK;
 }
 
@@ -344,13 +314,14 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
     // the ring, the copy stream and its events are the context's: one upload at
     // a time has them, until both streams are done with it
     std::unique_lock<std::mutex> staged(ctx->stage_lock, std::defer_lock);
-    void* staging = nullptr;  // a ring of slices too large to keep
+    void* stage = nullptr;  // the ring of slices
+    size_t stage_bytes = 0;
     const void* registered = nullptr;  // caller's host voxels registered for direct device reads
     cudaError_t e = cudaSuccess;
     auto cleanup = [&](vrc_status s, const std::string& m) {
         if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
         cudaStreamSynchronize(ctx->stream);
-        if (staging) cudaFree(staging);
+        if (stage) ctx->kept->put(vrc::KeptMemory::STAGE, stage, stage_bytes, VRC_STAGE_KEEP);
         if (registered) cudaHostUnregister(const_cast<void*>(registered));
         vrc_volume_destroy(v);
         return fail(ctx, s, m);
@@ -385,7 +356,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
     }
     const size_t pool = placement == VRC_PLACE_HOST ? 0 : (brick_bytes + 255) / 256 * 256;
     v->block_bytes = pool + floats * sizeof(float);
-    if (!(v->d_block = ctx->kept->take(v->block_bytes, &v->block_bytes)) &&
+    if (!(v->d_block = ctx->kept->take(vrc::KeptMemory::VOLUME, v->block_bytes, 2 * v->block_bytes, &v->block_bytes)) &&
         (e = vrc::device_alloc(*ctx->kept, &v->d_block, v->block_bytes)) != cudaSuccess)
         return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: brick pool and min/max table allocation failed");
     if (pool) v->d_bricks = v->d_block;
@@ -436,14 +407,9 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         const int layers = (int)std::min<size_t>(std::max<size_t>(VRC_SLAB_BYTES / (slice * L.B), 1), L.nb[2]);
         const int ring = (int)std::min<long long>(2ll * layers * L.B + vrc::APRON_LO + vrc::APRON_HI, Z);
         staged.lock();
-        char* stage = nullptr;
-        if (ring * slice <= VRC_STAGE_KEEP) {
-            e = ensure(ctx, &ctx->d_stage, &ctx->stage_bytes, ring * slice);
-            stage = (char*)ctx->d_stage;
-        } else {
-            e = vrc::device_alloc(*ctx->kept, &staging, ring * slice);
-            stage = (char*)staging;
-        }
+        stage_bytes = ring * slice;
+        if (!(stage = ctx->kept->take(vrc::KeptMemory::STAGE, stage_bytes, SIZE_MAX, &stage_bytes)))
+            e = vrc::device_alloc(*ctx->kept, &stage, stage_bytes);
         if (e != cudaSuccess) return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_upload: staging allocation failed");
         if (!ctx->copy_stream) e = cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking);
         for (cudaEvent_t* ev : {&ctx->copied[0], &ctx->copied[1], &ctx->consumed[0], &ctx->consumed[1], &ctx->queued})
@@ -460,7 +426,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             if (l0 >= 2 * layers) e = cudaStreamWaitEvent(ctx->copy_stream, ctx->consumed[k], 0);
             while (have < end && e == cudaSuccess) {
                 const int at = have % ring, n = std::min(end - have, ring - at);
-                e = cudaMemcpyAsync(stage + at * slice, (const char*)voxels + have * slice, n * slice, cudaMemcpyHostToDevice,
+                e = cudaMemcpyAsync((char*)stage + at * slice, (const char*)voxels + have * slice, n * slice, cudaMemcpyHostToDevice,
                                     ctx->copy_stream);
                 have += n;
             }
@@ -496,8 +462,7 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             cudaSuccess ||
         (e = cudaStreamSynchronize(ctx->stream)) != cudaSuccess)
         return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: ") + cudaGetErrorString(e));
-    if (staging) cudaFree(staging);
-    staging = nullptr;
+    if (stage) ctx->kept->put(vrc::KeptMemory::STAGE, stage, stage_bytes, VRC_STAGE_KEEP);
     if (registered) cudaHostUnregister(const_cast<void*>(registered));
     registered = nullptr;
     v->vmin = *std::min_element(mn.begin(), mn.end());
@@ -514,7 +479,7 @@ vrc_status vrc_volume_destroy(vrc_volume* v) {
     // are what cudaFree waits for. (Not a wait for the device here: it would
     // end any capture that another thread has under way.)
     if (v->d_block && v->kept && !v->off_stream.load())
-        v->kept->put(v->d_block, v->block_bytes);
+        v->kept->put(vrc::KeptMemory::VOLUME, v->d_block, v->block_bytes, VRC_VOLUME_KEEP);
     else
         cudaFree(v->d_block);
     if (v->h_bricks) cudaFreeHost(v->h_bricks);
@@ -727,9 +692,9 @@ vrc_status vrc_tf_create(vrc_context* ctx, const uint8_t* rgba, int width, float
     std::memcpy(t->h_rgba, rgba, 4 * width);
     std::vector<int> prefix(width + 1, 0);
     for (int i = 0; i < width; ++i) prefix[i + 1] = prefix[i] + (rgba[4 * i + 3] > 0 ? 1 : 0);
-    cudaError_t e = cudaMalloc(&t->d_prefix, (width + 1) * sizeof(int));
+    cudaError_t e = vrc::device_alloc(*ctx->kept, &t->d_prefix, (width + 1) * sizeof(int));
     if (e == cudaSuccess) e = cudaMemcpy(t->d_prefix, prefix.data(), (width + 1) * sizeof(int), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&t->d_rgba8, (size_t)width * 4);
+    if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &t->d_rgba8, (size_t)width * 4);
     if (e == cudaSuccess) e = cudaMemcpy(t->d_rgba8, rgba, (size_t)width * 4, cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
         vrc_tf_destroy(t);
@@ -839,7 +804,7 @@ vrc_status tf_alpha(vrc_context* ctx, vrc_tf* tf, bool corrected, float kcorr, f
     float h[256];
     tf_alpha_values(corrected, kcorr, h);
     float* d = nullptr;
-    cudaError_t e0 = cudaMalloc(&d, sizeof(h));
+    cudaError_t e0 = vrc::device_alloc(*ctx->kept, &d, sizeof(h));
     if (e0 != cudaSuccess) return cuda_fail(ctx, e0, "tf alpha table allocation");
     cudaError_t e = cudaMemcpy(d, h, sizeof(h), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) {
@@ -1020,7 +985,7 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
     const bool same_plan = vol->cache_valid && !vol->used_pending && vol->pending_pos >= vol->pending.size() &&
                            std::memcmp(src_key, vol->cache_src_key, sizeof(src_key)) == 0;
     if (!same_plan) {
-        if (!vol->d_occ_brick) VRC_CUDA(ctx, cudaMalloc((void**)&vol->d_occ_brick, words * 4));
+        if (!vol->d_occ_brick) VRC_CUDA(ctx, vrc::device_alloc(*ctx->kept, &vol->d_occ_brick, words * 4));
         VRC_CUDA(ctx, vrc::launch_occupancy(vol->d_bmin, vol->d_bmax, nb, occ_prefix, occ_width, vol->desc.rwm_scale,
                                             vol->desc.rwm_offset, tf->lo, tf->hi, vol->d_occ_brick, s));
         ++*launches;
@@ -1035,7 +1000,7 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
         const size_t brick_bytes = (size_t)L.brick_stride * vrc::dtype_bytes(vol->desc.dtype);
         if (vol->h_slot.size() != (size_t)nb) vol->h_slot.assign((size_t)nb, -1);
         if (vol->h_last_used.size() != (size_t)nb) vol->h_last_used.assign((size_t)nb, 0);
-        if (!vol->d_slot) VRC_CUDA(ctx, cudaMalloc((void**)&vol->d_slot, (size_t)nb * sizeof(int)));
+        if (!vol->d_slot) VRC_CUDA(ctx, vrc::device_alloc(*ctx->kept, &vol->d_slot, (size_t)nb * sizeof(int)));
         bool table_changed = false;
         if (!(vol->cache_valid && occ == vol->h_occ)) {
             // the slot table is uploaded whenever the cache is (re)planned: a new
@@ -1072,6 +1037,7 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
                 size_t free_b = 0, total_b = 0;
                 VRC_CUDA(ctx, cudaMemGetInfo(&free_b, &total_b));
                 const size_t reserve = (size_t)1 << 30;  // left for the frame buffers and other work
+                free_b += ctx->kept->held();              // which the allocation may have back
                 const long long fit = free_b > reserve ? (long long)((free_b - reserve) / brick_bytes) : 0;
                 slots = std::min(slots, fit + vol->cache_slots);
             }
@@ -1086,8 +1052,8 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
                 vol->free_slots.clear();
                 std::fill(vol->h_slot.begin(), vol->h_slot.end(), -1);
                 cudaError_t e = vrc::device_alloc(*ctx->kept, &vol->d_cache, (size_t)slots * brick_bytes);
-                if (e == cudaSuccess) e = cudaMalloc((void**)&vol->d_cache_ids, (size_t)slots * sizeof(long long));
-                if (e == cudaSuccess) e = cudaMalloc((void**)&vol->d_cache_dst, (size_t)slots * sizeof(long long));
+                if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &vol->d_cache_ids, (size_t)slots * sizeof(long long));
+                if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &vol->d_cache_dst, (size_t)slots * sizeof(long long));
                 if (e != cudaSuccess) {
                     cudaGetLastError();
                     cudaFree(vol->d_cache);
@@ -1196,7 +1162,7 @@ vrc_status prepare_brick_cache(vrc_context* ctx, vrc_volume* vol, const int* occ
         }
     }
     if (vol->cache_slots > 0 && (lod || resident < vol->cache_reachable)) {
-        if (!vol->d_used) VRC_CUDA(ctx, cudaMalloc((void**)&vol->d_used, words * 4));
+        if (!vol->d_used) VRC_CUDA(ctx, vrc::device_alloc(*ctx->kept, &vol->d_used, words * 4));
         VRC_CUDA(ctx, cudaMemsetAsync(vol->d_used, 0, words * 4, s));
         P.brick_used = vol->d_used;
         vol->used_pending = true;

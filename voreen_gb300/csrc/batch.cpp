@@ -168,8 +168,8 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
             const long long cells = (long long)nc[0] * nc[1] * nc[2];
             uint32_t* map = nullptr;
             uint8_t* dist = nullptr;
-            if ((e = vrc::device_alloc(*ctx->kept, (void**)&map, vrc::occupancy_bytes(cells))) == cudaSuccess) b->occ.push_back(map);
-            if (e == cudaSuccess && (e = vrc::device_alloc(*ctx->kept, (void**)&dist, (size_t)cells)) == cudaSuccess) b->dist.push_back(dist);
+            if ((e = vrc::device_alloc(*ctx->kept, &map, vrc::occupancy_bytes(cells))) == cudaSuccess) b->occ.push_back(map);
+            if (e == cudaSuccess && (e = vrc::device_alloc(*ctx->kept, &dist, (size_t)cells)) == cudaSuccess) b->dist.push_back(dist);
             if (e != cudaSuccess) {
                 release(b);
                 return bfail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_batch_create: occupancy allocation");
@@ -210,9 +210,9 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
         prefix[k + 1] = prefix[k] + (unsigned)t;
     }
     b->total_tiles = prefix[n];
-    if ((e = cudaMalloc((void**)&b->d_reqs, n * sizeof(vrc::BatchReq))) != cudaSuccess ||
-        (e = cudaMalloc((void**)&b->d_prefix, (n + 1) * sizeof(unsigned))) != cudaSuccess ||
-        (e = cudaMalloc((void**)&b->d_state, (3 + n) * sizeof(unsigned long long))) != cudaSuccess) {
+    if ((e = vrc::device_alloc(*ctx->kept, &b->d_reqs, n * sizeof(vrc::BatchReq))) != cudaSuccess ||
+        (e = vrc::device_alloc(*ctx->kept, &b->d_prefix, (n + 1) * sizeof(unsigned))) != cudaSuccess ||
+        (e = vrc::device_alloc(*ctx->kept, &b->d_state, (3 + n) * sizeof(unsigned long long))) != cudaSuccess) {
         release(b);
         return bfail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_batch_create: descriptor allocation");
     }
@@ -229,10 +229,8 @@ vrc_status create_batch(vrc_context* ctx, const vrc_batch_item* all, int n_items
         uint8_t* dist_tmp = nullptr;  // scratch of the distance passes, shared by the requests in turn
         size_t tmp_bytes = (size_t)max_cells;
         for (const Occ& j : occ_jobs) tmp_bytes = std::max(tmp_bytes, vrc::occ_distance_scratch(j.nc));
-        if ((e = vrc::device_alloc(*ctx->kept, (void**)&dist_tmp, tmp_bytes)) != cudaSuccess) {
-            cudaGetLastError();
-            e = vrc::device_alloc(*ctx->kept, (void**)&dist_tmp, tmp_bytes = (size_t)max_cells);
-        }
+        if ((e = vrc::device_alloc(*ctx->kept, &dist_tmp, tmp_bytes)) != cudaSuccess)
+            e = vrc::device_alloc(*ctx->kept, &dist_tmp, tmp_bytes = (size_t)max_cells);
         if (e != cudaSuccess) {
             release(b);
             return bfail(ctx, VRC_ERR_OUT_OF_MEMORY, "vrc_batch_create: distance scratch allocation");

@@ -32,9 +32,10 @@ extern "C" vrc_status vrc_occupancy_distance(vrc_context* ctx, const uint32_t* d
     if (n >= (1LL << 32)) return VRC_ERR_INVALID_ARG;
     const int nc[3] = {nx, ny, nz};
     uint8_t* tmp = nullptr;
-    const size_t bytes = std::max((size_t)n, vrc::occ_distance_scratch(nc));
+    size_t bytes = std::max((size_t)n, vrc::occ_distance_scratch(nc));
     cudaError_t e = cudaSetDevice(ctx->device);
-    if (e == cudaSuccess) e = cudaMalloc(&tmp, bytes);
+    if (e == cudaSuccess && (e = vrc::device_alloc(*ctx->kept, &tmp, bytes)) != cudaSuccess)
+        e = vrc::device_alloc(*ctx->kept, &tmp, bytes = (size_t)n);  // the passes take less
     if (e == cudaSuccess) e = vrc::launch_occ_distance(d_bits, nc, d_out, tmp, bytes, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(tmp);
@@ -53,8 +54,8 @@ extern "C" vrc_status vrc_measure_l2_read(vrc_context* ctx, size_t bytes, int re
     const int blocks = ctx->num_sms * 8, threads = 256;
     uint4 *buf = nullptr, *sink = nullptr;
     float ms = 0.f;
-    if (e == cudaSuccess) e = cudaMalloc(&buf, (size_t)n * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&sink, (size_t)blocks * threads * 16);
+    if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &buf, (size_t)n * 16);
+    if (e == cudaSuccess) e = vrc::device_alloc(*ctx->kept, &sink, (size_t)blocks * threads * 16);
     if (e == cudaSuccess) e = cudaMemsetAsync(buf, 1, (size_t)n * 16, ctx->stream);
     if (e == cudaSuccess) {
         l2_read_kernel<<<blocks, threads, 0, ctx->stream>>>(buf, n, 2, sink);  // bring the buffer into L2

@@ -290,7 +290,7 @@ vrc_status vrc_volume_load_vvd(vrc_context* ctx, const char* vvd_path, int brick
         return s == VRC_OK ? VRC_OK : ifail(ctx, s, m);
     };
     if (e != cudaSuccess) return cleanup(VRC_ERR_CUDA, "vrc_volume_load_vvd: cudaSetDevice");
-    if ((e = cudaMalloc(&d_lin, bytes)) != cudaSuccess)
+    if ((e = vrc::device_alloc(*ctx->kept, &d_lin, bytes)) != cudaSuccess)
         return cleanup(VRC_ERR_OUT_OF_MEMORY, "vrc_volume_load_vvd: device staging allocation");
     const size_t chunk = bytes < CHUNK ? bytes : CHUNK;
     for (int i = 0; i < 2; ++i) {

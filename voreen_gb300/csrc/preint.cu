@@ -145,8 +145,8 @@ vrc_status vrc_preint_create(vrc_context* ctx, const uint8_t* src, int res, floa
         delete t;
         return st;
     };
-    if ((e = cudaMalloc(&t->d_table, n * sizeof(float4))) != cudaSuccess) return bail(e, "pre-integration table");
-    if ((e = cudaMalloc(&t->d_prefix, (res + 1) * sizeof(int))) != cudaSuccess) return bail(e, "pre-integration prefix");
+    if ((e = vrc::device_alloc(*ctx->kept, &t->d_table, n * sizeof(float4))) != cudaSuccess) return bail(e, "pre-integration table");
+    if ((e = vrc::device_alloc(*ctx->kept, &t->d_prefix, (res + 1) * sizeof(int))) != cudaSuccess) return bail(e, "pre-integration prefix");
     if ((e = cudaMemcpyAsync(t->d_prefix, prefix.data(), (res + 1) * sizeof(int), cudaMemcpyHostToDevice, s)) !=
         cudaSuccess)
         return bail(e, "pre-integration prefix upload");
@@ -166,9 +166,9 @@ vrc_status vrc_preint_create(vrc_context* ctx, const uint8_t* src, int res, floa
             a8[i] = src[4 * i + 3];
             tb4[i] = make_float4(tb[i].r, tb[i].g, tb[i].b, tb[i].a);
         }
-        if ((e = cudaMalloc(&d_tb, res * sizeof(float4))) != cudaSuccess ||
-            (e = cudaMalloc(&d_a8, res)) != cudaSuccess ||
-            (e = cudaMalloc(&d_corr, corr.size() * sizeof(float))) != cudaSuccess)
+        if ((e = vrc::device_alloc(*ctx->kept, &d_tb, res * sizeof(float4))) != cudaSuccess ||
+            (e = vrc::device_alloc(*ctx->kept, &d_a8, res)) != cudaSuccess ||
+            (e = vrc::device_alloc(*ctx->kept, &d_corr, corr.size() * sizeof(float))) != cudaSuccess)
             return bail(e, "pre-integration scratch");
         if ((e = cudaMemcpyAsync(d_tb, tb4.data(), res * sizeof(float4), cudaMemcpyHostToDevice, s)) != cudaSuccess ||
             (e = cudaMemcpyAsync(d_a8, a8.data(), res, cudaMemcpyHostToDevice, s)) != cudaSuccess ||

@@ -330,8 +330,14 @@ void CudaRaycaster::process(bool analytic, bool interacting) {
         p.entry_exit_mode = VRC_EE_ANALYTIC;
         void* small = nullptr;
         void* full = nullptr;
-        cudaError_t e = cudaMalloc(&small, (size_t)p.width * p.height * 16);
-        if (e == cudaSuccess) e = cudaMalloc(&full, (size_t)W * H * 16);
+        auto alloc = [&](void** image, size_t bytes) {
+            cudaError_t r = cudaMalloc(image, bytes);
+            if (r == cudaErrorMemoryAllocation && vrc_context_trim(ctx_) == VRC_OK) r = cudaMalloc(image, bytes);
+            if (r != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch
+            return r;
+        };
+        cudaError_t e = alloc(&small, (size_t)p.width * p.height * 16);
+        if (e == cudaSuccess) e = alloc(&full, (size_t)W * H * 16);
         bool ok = e == cudaSuccess;
         if (!ok) error(std::string("interaction buffers: ") + cudaGetErrorString(e));
         ok = ok && check(vrc_render(ctx_, vol_, tf, &p, nullptr, nullptr, 0, small, VRC_OUT_RGBA32F, 1, &lastStats),

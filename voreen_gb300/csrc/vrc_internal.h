@@ -228,24 +228,39 @@ size_t occ_distance_scratch(const int nc[3]);
 int occ_distance_launches(const int nc[3], size_t tmp_bytes);
 inline size_t occupancy_bytes(long long ncells) { return (size_t)((ncells + 31) / 32) * 4; }
 
-// The memory of the last volume of a context that was destroyed, up to
-// VRC_VOLUME_KEEP bytes, for the next one of about its size. Volumes may be
-// destroyed by any thread, and after their context.
-struct KeptBlock {
-    std::mutex lock;
-    void* p = nullptr;
-    size_t bytes = 0;
-    bool closed = false;  // the context is gone
+// Device memory that a context keeps between calls: the block of the last
+// volume destroyed, for the next one of about its size, and the slices of host
+// voxels on their way in. Volumes may be destroyed by any thread, and after
+// their context. All of it goes back when an allocation of the context finds no
+// memory (device_alloc), on vrc_context_trim, and with the context.
+class KeptMemory {
+public:
+    enum Kind { VOLUME, STAGE, KINDS };
+    // the kept block if it holds `need` bytes and at most `most`: the caller's from here on
+    void* take(Kind k, size_t need, size_t most, size_t* got);
+    // keeps a block of up to `limit` bytes, in the place of the one kept
+    // before, or frees it. Only work on the context's stream, or work that has
+    // been waited for, has used it.
+    void put(Kind k, void* p, size_t bytes, size_t limit);
+    // frees what is kept; false if there was nothing. close: and keeps nothing more
+    bool give_back(bool close = false);
+    size_t held();
     int device = 0;
-    // the block if it holds `need` bytes and not over twice as many
-    void* take(size_t need, size_t* got);
-    // keeps a block that only work on the context's stream has used, or frees it
-    void put(void* block, size_t n);
-    // frees what is kept; false if there was nothing
-    bool give_back(bool close);
+
+private:
+    struct Block {
+        void* p = nullptr;
+        size_t bytes = 0;
+    };
+    std::mutex lock;
+    Block blocks[KINDS];
+    bool closed = false;  // the context is gone
 };
-// Device memory, giving the kept block back where there is none left.
-cudaError_t device_alloc(KeptBlock& kept, void** p, size_t bytes);
+// Device memory; where there is none left, what the context keeps is given back first.
+cudaError_t device_alloc_bytes(KeptMemory& kept, void** p, size_t bytes);
+template <typename T> cudaError_t device_alloc(KeptMemory& kept, T** p, size_t bytes) {
+    return device_alloc_bytes(kept, reinterpret_cast<void**>(p), bytes);
+}
 
 // Process-unique id of a volume, TF or pre-integration table: identifies
 // the derived data cached for it even when an address is reused later.
@@ -275,10 +290,8 @@ struct vrc_context {
     uint8_t* d_dist = nullptr;       // occ_dist of the skip cells, and the passes' scratch
     uint8_t* d_dist_tmp = nullptr;
     size_t dist_bytes = 0, dist_tmp_bytes = 0;
-    void* d_stage = nullptr;         // slices of a volume on their way in, up to VRC_STAGE_KEEP bytes
-    size_t stage_bytes = 0;
-    std::mutex stage_lock;           // the upload that has them and the copy stream
-    std::shared_ptr<vrc::KeptBlock> kept = std::make_shared<vrc::KeptBlock>();
+    std::shared_ptr<vrc::KeptMemory> kept;
+    std::mutex stage_lock;           // the upload that has the kept slices, the copy stream and its events
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr}, queued = nullptr;
     int* d_prefix = nullptr;
@@ -340,7 +353,7 @@ struct vrc_volume {
     vrc::BrickLayout lod_L{};
     int lod_level = 0;                 // level d_lod holds: 1 = half resolution, k = 2^-k
     bool lod_on = false;
-    std::shared_ptr<vrc::KeptBlock> kept;  // the context's
+    std::shared_ptr<vrc::KeptMemory> kept;  // the context's
     void* d_block = nullptr;  // the allocation of the brick pool (device placement) and all min/max tables
     size_t block_bytes = 0;
     mutable std::atomic<bool> off_stream{false};  // a frame went to a stream of the caller's
@@ -366,8 +379,7 @@ struct vrc_volume {
 #define VRC_SLAB_BYTES (56u << 20)
 #endif
 // The largest block of a destroyed volume that a context keeps: cudaMalloc and
-// cudaFree of 512^3 u16's 505 MB took 640 us a new time step of 2990. Given back to the next volume, on
-// the first allocation that finds no memory, and with the context.
+// cudaFree of 512^3 u16's 505 MB took 640 us a new time step of 2990.
 #ifndef VRC_VOLUME_KEEP
 #define VRC_VOLUME_KEEP (1u << 30)
 #endif
