@@ -107,8 +107,9 @@ vrc_status vrc_context_create(int device, vrc_context** out);
 vrc_status vrc_context_destroy(vrc_context* ctx);
 vrc_status vrc_context_synchronize(vrc_context* ctx);
 /* Between calls a context keeps the device memory of the last volume destroyed,
- * up to 1 GiB, for its next volume of about that size, and up to 128 MB of
- * staging for host voxels. It gives them back when one of its own allocations
+ * up to 1 GiB, for its next volume of about that size, up to 128 MB of staging
+ * for host voxels, and the scratch that an empty-space map is built with (2
+ * bytes a cell, or a little more where rows are no multiple of 32 cells). It gives them back when one of its own allocations
  * finds no memory, when it is destroyed, and here: for callers whose other
  * allocations on the device need the room. */
 vrc_status vrc_context_trim(vrc_context* ctx);

@@ -108,6 +108,36 @@ int main() {
     }
     {
         K kept;
+        void* p = nullptr;
+        size_t got = 0;
+        auto use = [&](size_t best, size_t least) {
+            mallocs = 0;
+            p = nullptr;
+            const cudaError_t e = kept.scratch(best, least, &p, &got);
+            assert(last == cudaSuccess);
+            if (e == cudaSuccess) kept.put(K::SCRATCH, p, got, SIZE_MAX);
+            return e;
+        };
+        room = 1000;
+        assert(use(400, 200) == cudaSuccess && got == 400 && mallocs == 1);
+        assert(use(400, 200) == cudaSuccess && got == 400 && mallocs == 0);  // again: nothing allocated
+        assert(use(100, 50) == cudaSuccess && got == 400 && mallocs == 0);
+        assert(use(900, 450) == cudaSuccess && got == 900 && mallocs == 1);  // beside the 400 it would not fit
+        assert(use(1200, 600) == cudaSuccess && got == 600 && mallocs == 2);  // refused: the smaller one
+        assert(use(1200, 600) == cudaSuccess && got == 600 && mallocs == 0);  // and not asked for again
+        assert(use(1200, 600) == cudaSuccess && got == 600 && mallocs == 0);
+        assert(use(2400, 1100) == cudaErrorMemoryAllocation && kept.held() == 0);
+        assert(use(1200, 600) == cudaSuccess && got == 600);
+        room += 1000;
+        assert(use(1200, 600) == cudaSuccess && got == 600 && mallocs == 0);
+        kept.give_back();  // room may have been made since
+        assert(use(1200, 600) == cudaSuccess && got == 1200 && mallocs == 1);
+        kept.give_back(true);
+        assert(live.empty());
+        room = SIZE_MAX;
+    }
+    {
+        K kept;
         std::vector<std::thread> threads;
         for (int t = 0; t < 4; ++t)
             threads.emplace_back([&kept, t] {

@@ -141,6 +141,29 @@ def test_failing_allocations_give_the_memory_back(vrc_lib, tmp_path):
     ctx.close()
 
 
+def test_scratch_of_the_maps_is_taken_only_to_build_them(vrc_lib):
+    """Frames whose maps are there take no scratch; one that builds them takes it
+    again after it was given back: the same image each time."""
+    ctx = v.Context(0)
+    vol = _volume(ctx, 512)
+    p = v.default_params(64, 48)
+    pos, focus, near, far = synth.orbit_camera(vol.dims, (1.0, 1.0, 1.0), 30.0, 20.0, 1.1)
+    p.camera, p.entry_exit_mode = v.make_camera(pos, focus, near=near, far=far), v.EE_ANALYTIC
+    tfs = [v.TransferFunction(ctx, v.TransferFunction.bake([(0.0, (0, 0, 0, 0)), (1.0, (255, 200, 100, 60))], 256), (0.0, 1.0))
+           for _ in range(2)]
+    first = np.array(v.render(ctx, vol, tfs[0], p, out_format=v.OUT_RGBA32F)[0])
+    held = _free()
+    ctx.trim()
+    trimmed = _free()
+    assert trimmed - held >= 30 * MIB  # 2^24 cells
+    np.testing.assert_array_equal(v.render(ctx, vol, tfs[0], p, out_format=v.OUT_RGBA32F)[0], first)
+    assert _free() >= trimmed - MIB
+    np.testing.assert_array_equal(v.render(ctx, vol, tfs[1], p, out_format=v.OUT_RGBA32F)[0], first)
+    assert _free() < trimmed - 16 * MIB
+    for x in (*tfs, vol, ctx):
+        x.close()
+
+
 def test_memory_returns_with_the_context_whoever_goes_first(vrc_lib):
     """A context closed before its volumes, and one after: nothing stays."""
     import torch

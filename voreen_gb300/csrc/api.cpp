@@ -244,7 +244,6 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_occ);
     cudaFree(c->d_occ_coarse);
     cudaFree(c->d_dist);
-    cudaFree(c->d_dist_tmp);
     c->kept->give_back(true);
     for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1], c->queued})
         if (ev) cudaEventDestroy(ev);
@@ -1314,15 +1313,7 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         const uint32_t* coarse_before = ctx->d_occ_coarse;
         const uint8_t* dist_before = ctx->d_dist;
         VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_occ, &ctx->occ_bytes, vrc::occupancy_bytes(n)));
-        if (use_dist) {
-            VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_dist, &ctx->dist_bytes, (size_t)n));
-            // the passes take less scratch where the planes' does not fit
-            if (ensure(ctx, (void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes,
-                       std::max((size_t)n, vrc::occ_distance_scratch(nc))) != cudaSuccess) {
-                cudaGetLastError();
-                VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_dist_tmp, &ctx->dist_tmp_bytes, (size_t)n));
-            }
-        }
+        if (use_dist) VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_dist, &ctx->dist_bytes, (size_t)n));
         if (use_coarse)
             VRC_CUDA(ctx, ensure(ctx, (void**)&ctx->d_occ_coarse, &ctx->occ_coarse_bytes,
                                  vrc::occupancy_bytes(vol->L.nbricks())));
@@ -1349,8 +1340,14 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
         P.skip_margin = 0.01f + 2e-5f * float(maxdim);
         if (use_dist) {
             if (!cached) {
-                VRC_CUDA(ctx, vrc::launch_occ_distance(ctx->d_occ, nc, ctx->d_dist, ctx->d_dist_tmp, ctx->dist_tmp_bytes, s));
-                occ_launches += vrc::occ_distance_launches(nc, ctx->dist_tmp_bytes);
+                // the passes take less scratch where the planes' does not fit
+                void* tmp = nullptr;
+                size_t bytes = 0;
+                VRC_CUDA(ctx, ctx->kept->scratch(std::max((size_t)n, vrc::occ_distance_scratch(nc)), (size_t)n, &tmp, &bytes));
+                const cudaError_t e = vrc::launch_occ_distance(ctx->d_occ, nc, ctx->d_dist, (uint8_t*)tmp, bytes, s);
+                ctx->kept->put(vrc::KeptMemory::SCRATCH, tmp, bytes, SIZE_MAX);
+                VRC_CUDA(ctx, e);
+                occ_launches += vrc::occ_distance_launches(nc, bytes);
             }
             P.occ_dist = ctx->d_dist;
         }

@@ -28,11 +28,38 @@ void KeptMemory::put(Kind k, void* p, size_t bytes, size_t limit) {
     cudaFree(p);
 }
 
+cudaError_t KeptMemory::scratch(size_t best, size_t least, void** p, size_t* got) {
+    void* small = nullptr;  // freed first: beside it the larger one might not fit
+    bool ask;
+    {
+        std::lock_guard<std::mutex> g(lock);
+        Block& b = blocks[SCRATCH];
+        ask = best != refused;
+        if (b.p && b.bytes >= (ask ? best : least)) {
+            *p = b.p;
+            *got = b.bytes;
+            b = Block{};
+            return cudaSuccess;
+        }
+        std::swap(small, b.p);
+        b = Block{};
+    }
+    cudaFree(small);
+    if (ask) {
+        const cudaError_t e = device_alloc_bytes(*this, p, *got = best);
+        if (e != cudaErrorMemoryAllocation) return e;
+        std::lock_guard<std::mutex> g(lock);
+        refused = best;
+    }
+    return device_alloc_bytes(*this, p, *got = least);
+}
+
 bool KeptMemory::give_back(bool close) {
     Block all[KINDS];
     {
         std::lock_guard<std::mutex> g(lock);
         std::swap(all, blocks);
+        refused = 0;
         closed = closed || close;
     }
     bool any = false;

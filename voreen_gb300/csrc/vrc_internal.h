@@ -229,19 +229,22 @@ int occ_distance_launches(const int nc[3], size_t tmp_bytes);
 inline size_t occupancy_bytes(long long ncells) { return (size_t)((ncells + 31) / 32) * 4; }
 
 // Device memory that a context keeps between calls: the block of the last
-// volume destroyed, for the next one of about its size, and the slices of host
-// voxels on their way in. Volumes may be destroyed by any thread, and after
-// their context. All of it goes back when an allocation of the context finds no
+// volume destroyed, for the next one of about its size, the slices of host
+// voxels on their way in, and the distance field's scratch. Volumes may be
+// destroyed by any thread, and after their context. All of it goes back when an allocation of the context finds no
 // memory (device_alloc), on vrc_context_trim, and with the context.
 class KeptMemory {
 public:
-    enum Kind { VOLUME, STAGE, KINDS };
+    enum Kind { VOLUME, STAGE, SCRATCH, KINDS };
     // the kept block if it holds `need` bytes and at most `most`: the caller's from here on
     void* take(Kind k, size_t need, size_t most, size_t* got);
     // keeps a block of up to `limit` bytes, in the place of the one kept
     // before, or frees it. Only work on the context's stream, or work that has
     // been waited for, has used it.
     void put(Kind k, void* p, size_t bytes, size_t limit);
+    // scratch of `best` bytes, or of `least` where that was refused; a size
+    // refused is not asked for again before memory was given back. To be put back.
+    cudaError_t scratch(size_t best, size_t least, void** p, size_t* got);
     // frees what is kept; false if there was nothing. close: and keeps nothing more
     bool give_back(bool close = false);
     size_t held();
@@ -254,6 +257,7 @@ private:
     };
     std::mutex lock;
     Block blocks[KINDS];
+    size_t refused = 0;
     bool closed = false;  // the context is gone
 };
 // Device memory; where there is none left, what the context keeps is given back first.
@@ -287,9 +291,8 @@ struct vrc_context {
     size_t occ_bytes = 0;
     uint32_t* d_occ_coarse = nullptr;
     size_t occ_coarse_bytes = 0;
-    uint8_t* d_dist = nullptr;       // occ_dist of the skip cells, and the passes' scratch
-    uint8_t* d_dist_tmp = nullptr;
-    size_t dist_bytes = 0, dist_tmp_bytes = 0;
+    uint8_t* d_dist = nullptr;       // occ_dist of the skip cells
+    size_t dist_bytes = 0;
     std::shared_ptr<vrc::KeptMemory> kept;
     std::mutex stage_lock;           // the upload that has the kept slices, the copy stream and its events
     cudaStream_t copy_stream = nullptr;
