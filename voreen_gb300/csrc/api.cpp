@@ -372,14 +372,16 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
             lv.d_min = take(lv.count());
             lv.d_max = take(lv.count());
         }
-    // bricks and finest cells of brick layers [l0, l1), whose slices are in `lin`
+    // bricks and finest cells of brick layers [l0, l1), whose slices are in
+    // `lin`; the bricks are the finest cells where half a brick's edge makes
+    // more than a level may have
+    const int C = finest ? finest->C : L.B;
+    float *const cmin = finest ? finest->d_min : v->d_bmin, *const cmax = finest ? finest->d_max : v->d_bmax;
     auto ingest = [&](const vrc::Slices& lin, int l0, int l1) {
+        const int per = L.B / C, ncz = (desc->dims[2] + C - 1) / C;
         cudaError_t r = vrc::launch_brick_build(lin, desc->dtype, L, l0, l1, v->d_bricks, ctx->stream);
-        if (r == cudaSuccess && finest) {
-            const int per = L.B / finest->C;
-            r = vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, finest->C, l0 * per, std::min(l1 * per, finest->nc[2]),
-                                        finest->d_min, finest->d_max, ctx->stream);
-        }
+        if (r == cudaSuccess)
+            r = vrc::launch_cell_minmax(lin, desc->dtype, desc->dims, C, l0 * per, std::min(l1 * per, ncz), cmin, cmax, ctx->stream);
         return r;
     };
     if (on_device) {
@@ -443,17 +445,12 @@ vrc_status vrc_volume_upload_placed(vrc_context* ctx, const vrc_volume_desc* des
         if (lv.d_max && fine.d_max)
             e = vrc::launch_coarser_minmax(fine.d_min, fine.d_max, fine.nc, 2, lv.nc, lv.d_min, lv.d_max, ctx->stream);
     }
+    // the bricks' from the coarsest cells (half a brick, or a quarter of a 64^3 one)
+    for (const auto& lv : v->levels)
+        if (e == cudaSuccess && lv.d_max && (lv.C * 2 == L.B || (lv.C * 4 == L.B && L.B == 64)))
+            e = vrc::launch_coarser_minmax(lv.d_min, lv.d_max, lv.nc, L.B / lv.C, L.nb, v->d_bmin, v->d_bmax, ctx->stream);
     if (e != cudaSuccess)
         return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: kernel: ") + cudaGetErrorString(e));
-    // the bricks' from the coarsest cells (half a brick, or a quarter of a 64^3 one)
-    const vrc_cell_level* half = nullptr;
-    for (const auto& lv : v->levels)
-        if (lv.d_max && (lv.C * 2 == L.B || (lv.C * 4 == L.B && L.B == 64))) half = &lv;
-    e = half ? vrc::launch_coarser_minmax(half->d_min, half->d_max, half->nc, L.B / half->C, L.nb, v->d_bmin, v->d_bmax,
-                                          ctx->stream)
-             : vrc::launch_brick_minmax(v->d_bricks, desc->dtype, L, v->d_bmin, v->d_bmax, ctx->stream);
-    if (e != cudaSuccess)
-        return cleanup(VRC_ERR_CUDA, std::string("vrc_volume_upload: brick kernel: ") + cudaGetErrorString(e));
     std::vector<float> mn(L.nbricks()), mx(L.nbricks());
     if ((e = cudaMemcpyAsync(mn.data(), v->d_bmin, mn.size() * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream)) !=
             cudaSuccess ||

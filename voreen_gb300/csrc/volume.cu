@@ -104,46 +104,6 @@ __global__ void half_sample_kernel(const T* __restrict__ bricks, BrickLayout L, 
     }
 }
 
-// One CTA per brick: min/max of the stored values over local [APRON_LO,
-// APRON_LO + B] on each axis (core + one voxel on the high side), i.e. the
-// voxels any trilinear stencil whose floor lies in the brick can touch.
-template <typename T>
-__global__ void brick_minmax_kernel(const T* __restrict__ bricks, BrickLayout L, float norm, float* bmin,
-                                    float* bmax) {
-    const long long b = blockIdx.x;
-    const T* base = bricks + b * L.brick_stride;
-    const int E = L.B + 1;
-    float mn = INFINITY, mx = -INFINITY;
-    for (int i = threadIdx.x; i < E * E * E; i += blockDim.x) {
-        const int x = i % E + APRON_LO, y = (i / E) % E + APRON_LO, z = i / (E * E) + APRON_LO;
-        const float v = raw_to_float(base[(z * L.S + y) * L.S + x]);
-        mn = fminf(mn, v);
-        mx = fmaxf(mx, v);
-    }
-    __shared__ float smn[32], smx[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { smn[w] = mn; smx[w] = mx; }
-    __syncthreads();
-    if (w == 0) {
-        const int nw = blockDim.x >> 5;
-        mn = lane < nw ? smn[lane] : INFINITY;
-        mx = lane < nw ? smx[lane] : -INFINITY;
-        for (int o = 16; o > 0; o >>= 1) {
-            mn = fminf(mn, __shfl_xor_sync(0xffffffffu, mn, o));
-            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        }
-        if (lane == 0) {
-            // getTypeAsFloat: value / rangeMax, correctly rounded (monotone)
-            bmin[b] = norm > 0.f ? __fdiv_rn(mn, norm) : mn;
-            bmax[b] = norm > 0.f ? __fdiv_rn(mx, norm) : mx;
-        }
-    }
-}
-
 // One thread per cell: min/max over the cell's voxels plus one voxel on the
 // high side of every axis (clamped), i.e. the trilinear support of all
 // samples whose floor voxel lies in the cell. Any cell edge and row length.
@@ -706,25 +666,6 @@ cudaError_t launch_half_sample(const void* bricks, int dtype, const BrickLayout&
         default:
             half_sample_kernel<float><<<g, 256, 0, s>>>((const float*)bricks, L, dims1[0], dims1[1], dims1[2],
                                                         (float*)out);
-            break;
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_brick_minmax(const void* bricks, int dtype, const BrickLayout& L, float* bmin, float* bmax,
-                                cudaStream_t s) {
-    const long long n = L.nbricks();
-    if (n > 0x7fffffffLL) return cudaErrorInvalidValue;
-    switch (dtype) {
-        case VRC_U8:
-            brick_minmax_kernel<uint8_t><<<(unsigned)n, 256, 0, s>>>((const uint8_t*)bricks, L, 255.f, bmin, bmax);
-            break;
-        case VRC_U16:
-            brick_minmax_kernel<uint16_t><<<(unsigned)n, 256, 0, s>>>((const uint16_t*)bricks, L, 65535.f, bmin,
-                                                                      bmax);
-            break;
-        default:
-            brick_minmax_kernel<float><<<(unsigned)n, 256, 0, s>>>((const float*)bricks, L, 0.f, bmin, bmax);
             break;
     }
     return cudaGetLastError();

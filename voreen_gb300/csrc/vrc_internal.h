@@ -203,8 +203,6 @@ cudaError_t launch_brick_build(const Slices& linear, int dtype, const BrickLayou
 // integers summed exactly and divided by 8 with truncation.
 cudaError_t launch_half_sample(const void* bricks, int dtype, const BrickLayout& L, const int dims1[3], void* out,
                                cudaStream_t s);
-cudaError_t launch_brick_minmax(const void* bricks, int dtype, const BrickLayout& L, float* bmin, float* bmax,
-                                cudaStream_t s);
 // Min/max of normalised intensity per cell of edge C over the cell's voxels
 // plus one voxel on the high side (clamped), from the linear volume; cells
 // [cz0, cz1) along z.
