@@ -15,6 +15,7 @@
 
 #include "../../include/vrc_nn.h"
 #include "nn_launch.cuh"
+#include "nn_rows.h"
 
 namespace {
 
@@ -425,8 +426,8 @@ __global__ void avgpool_kernel(const __nv_bfloat16* in, int rows, int H, int W, 
     };
     const int Ho = H / 2, Wo = W / 2, CV = C / V;
     after_previous();
-    for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
-        const int b = row / Ho, y = row - b * Ho;
+    for (long long at_row = blockIdx.y; at_row < rows; at_row += gridDim.y) {  // the images' output rows; past them it may pass an int
+        const int row = (int)at_row, b = row / Ho, y = row - b * Ho;
         const Vec* p = reinterpret_cast<const Vec*>(in + ((size_t)b * H + 2 * y) * W * C);
         const Vec* q = p + (size_t)W * CV;
         Vec* o = reinterpret_cast<Vec*>(out + (size_t)row * Wo * C);
@@ -507,13 +508,14 @@ __device__ __forceinline__ float4 bilerp_base4(const float4* p, int H, int W, in
 }
 __global__ void __launch_bounds__(128) head_fwd_kernel(const float4* feat4, const float4* base, int rows, int H, int W, float4* out) {
     const int Ho = 2 * H, Wo = 2 * W;
+    const unsigned ox = blockIdx.x * 128u + threadIdx.x;  // the grid covers a row
     after_previous();
-    for (int row = blockIdx.y; row < rows; row += gridDim.y) {  // N * Ho output rows
-        const int b = row / Ho, oy = row - b * Ho;
+    for (long long at_row = blockIdx.y; at_row < rows; at_row += gridDim.y) {  // the images' output rows; past them it may pass an int
+        const int row = (int)at_row, b = row / Ho, oy = row - b * Ho;
         const float4* f4 = feat4 + ((size_t)b * H + oy / 2) * W * 4 + 2 * (oy & 1);
-        for (int ox = blockIdx.x * 128 + threadIdx.x; ox < Wo; ox += gridDim.x * 128) {
+        if (ox < (unsigned)Wo) {
             const float4 f = f4[(size_t)(ox >> 1) * 4 + (ox & 1)];
-            const float4 u = bilerp_base4(base + (size_t)b * H * W, H, W, oy, ox);
+            const float4 u = bilerp_base4(base + (size_t)b * H * W, H, W, oy, (int)ox);
             out[(size_t)row * Wo + ox] = make_float4(f.x + u.x, f.y + u.y, f.z + u.z, f.w + u.w);
         }
     }
@@ -792,16 +794,20 @@ int vrc_nn_relu_bwd(const void* y, void* dy, long long n, int leaky, void* strea
 
 int vrc_nn_avgpool2(const void* in, int N, int H, int W, int C, float scale, void* out, void* stream) {
     if (H % 2 || W % 2) return 1;
-    const int rows = N * (H / 2);
     const bool wide = C % 8 == 0 && (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0;
     const long long per_row = (long long)(W / 2) * (wide ? C / 8 : C);
-    const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>((per_row + 255) / 256, 65535)),
-                    (unsigned)std::max(1, std::min(rows, 65535)));
-    const auto* i = static_cast<const __nv_bfloat16*>(in);
-    auto* o = static_cast<__nv_bfloat16*>(out);
-    if (wide)
-        return status_of(launch_chained(avgpool_kernel<8>, grid, 256, 0, static_cast<cudaStream_t>(stream), i, rows, H, W, C, scale, o));
-    return status_of(launch_chained(avgpool_kernel<1>, grid, 256, 0, static_cast<cudaStream_t>(stream), i, rows, H, W, C, scale, o));
+    const int images = images_per_launch(N, H / 2);
+    cudaError_t e = cudaSuccess;
+    for (long long n = 0; n < std::max(N, 1) && e == cudaSuccess; n += images) {
+        const int rows = (int)std::min<long long>(N - n, images) * (H / 2);
+        const dim3 grid((unsigned)std::max<long long>(1, std::min<long long>((per_row + 255) / 256, 65535)),
+                        (unsigned)std::max(1, std::min(rows, 65535)));
+        const auto* i = static_cast<const __nv_bfloat16*>(in) + (size_t)n * H * W * C;
+        auto* o = static_cast<__nv_bfloat16*>(out) + (size_t)n * (H / 2) * (W / 2) * C;
+        e = launch_chained(wide ? avgpool_kernel<8> : avgpool_kernel<1>, grid, 256, 0, static_cast<cudaStream_t>(stream), i, rows,
+                           H, W, C, scale, o);
+    }
+    return status_of(e);
 }
 
 int vrc_nn_upsample2(const void* in, int N, int H, int W, int C, float scale, void* out, void* stream) {
@@ -825,15 +831,20 @@ int vrc_nn_add(void* a, const void* b, long long n, void* stream) {
 
 int vrc_nn_head_fwd(const float* feat16, const float* base, int N, int H, int W, float* out, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int rows = 2 * N * H;
     if ((reinterpret_cast<uintptr_t>(feat16) | reinterpret_cast<uintptr_t>(base) | reinterpret_cast<uintptr_t>(out)) % 16) {
         head_fwd_unaligned_kernel<<<ew_grid((long long)N * H * W * 16), 256, 0, st>>>(feat16, base, N, H, W, out);
-    } else {
-        const dim3 grid((unsigned)std::max(1, (2 * W + 127) / 128), (unsigned)std::max(1, std::min(rows, 65535)));
-        return status_of(launch_chained(head_fwd_kernel, grid, 128, 0, st, reinterpret_cast<const float4*>(feat16),
-                                        reinterpret_cast<const float4*>(base), rows, H, W, reinterpret_cast<float4*>(out)));
+        return status_of(cudaGetLastError());
     }
-    return status_of(cudaGetLastError());
+    const int images = images_per_launch(N, 2ll * H);
+    cudaError_t e = cudaSuccess;
+    for (long long n = 0; n < std::max(N, 1) && e == cudaSuccess; n += images) {
+        const int rows = (int)std::min<long long>(N - n, images) * 2 * H;
+        const dim3 grid((unsigned)std::max(1ll, (2ll * W + 127) / 128), (unsigned)std::max(1, std::min(rows, 65535)));
+        const size_t pixels = (size_t)n * H * W;  // before these images
+        e = launch_chained(head_fwd_kernel, grid, 128, 0, st, reinterpret_cast<const float4*>(feat16) + 4 * pixels,
+                           reinterpret_cast<const float4*>(base) + pixels, rows, H, W, reinterpret_cast<float4*>(out) + 4 * pixels);
+    }
+    return status_of(e);
 }
 
 int vrc_nn_head_bwd(const float* dout, int N, int H, int W, void* dfeat16, void* stream) {
