@@ -141,6 +141,26 @@ def test_failing_allocations_give_the_memory_back(vrc_lib, tmp_path):
     ctx.close()
 
 
+def test_a_refused_frame_does_not_count_as_one_on_another_stream(vrc_lib):
+    """Volumes too large for vrc_render_noalloc's scratch (the learned form's
+    probe asks first) leave their memory to the next volume, like others."""
+    import torch
+    ctx = v.Context(0)
+    vol = _volume(ctx, 512)
+    p = v.default_params(32, 32)
+    p.entry_exit_mode, p.skip_cell_size = v.EE_ANALYTIC, 2
+    p.camera = v.make_camera((256, 256, 1500), (256, 256, 256), near=1.0, far=3000.0)
+    tf = v.TransferFunction(ctx, v.TransferFunction.bake([(0.0, (0, 0, 0, 0)), (1.0, (255, 255, 255, 255))], 256))
+    with pytest.raises(v.VrcError) as ei:
+        v.render_noalloc(vol, tf, p, None, None, torch.zeros((32, 32, 4), device="cuda"), v.OUT_RGBA32F, ctx.stream)
+    assert ei.value.status == 8
+    tf.close()
+    before = _free()
+    vol.close()
+    assert _free() - before < MIB
+    ctx.close()
+
+
 def test_scratch_of_the_maps_is_taken_only_to_build_them(vrc_lib):
     """Frames whose maps are there take no scratch; one that builds them takes it
     again after it was given back: the same image each time."""

@@ -93,7 +93,6 @@ struct DeviceScope {
 
 vrc_status render_noalloc(const vrc_volume* vol, const vrc_tf* tf, const vrc_render_params* p, const float* d_entry,
                           const float* d_exit, void* d_out, int out_format, cudaStream_t s, int dev) {
-    vol->off_stream.store(true);
     unsigned char* scratch = static_cast<unsigned char*>(g_scratch_addr[dev]);
     vrc::MarchParams P;
     vrc_status st = vrc::fill_params(nullptr, vol, p, P);
@@ -121,6 +120,7 @@ vrc_status render_noalloc(const vrc_volume* vol, const vrc_tf* tf, const vrc_ren
         }
     const long long ncells = (long long)nc[0] * nc[1] * nc[2];
     if (p->empty_space_skipping && ncells > (long long)VRC_NOALLOC_MAX_CELLS) return VRC_ERR_SCRATCH_LIMIT;
+    vol->off_stream.store(true);  // from here on the caller's stream reads the volume
 
     // The TF's RGBA8 entries are read where the TF object keeps them on the
     // device; its alpha per alpha byte (vrc_render's host arithmetic) goes into
