@@ -328,12 +328,10 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
         const __nv_bfloat16 *s_d = smem + set * WT::STAGE, *s_i = s_d + WT::D;
         // Where the tile overhangs the image on the right, the image's last
         // column is staged for kw = 1 and 2, but its output pixel at kw = 0
-        // lies outside: out of that operand (pixels 2t, 2t + 1 and + 8 in this
-        // thread's registers), as 0 times an infinity would not be 0. Rows and
-        // the columns beyond it are zeros already.
-        const int over = W - (tile % tiles_x) * 16 - 2 * (lane & 3);
-        const uint32_t keep0 = over == 0 ? 0xffff0000u : over == 1 ? 0x0000ffffu : ~0u;
-        const uint32_t keep8 = over == 8 ? 0xffff0000u : over == 9 ? 0x0000ffffu : ~0u;
+        // lies outside, and 0 times an infinity is not 0: there this lane's row
+        // of that operand is column 17, zeros. Rows and the columns beyond it
+        // are zeros already.
+        const int px = ((lane >> 3) & 1) * 8 + (lane & 7), px0 = px == W - (tile % tiles_x) * 16 ? 17 : px;
         if (sums_bias)
             for (int p = tid / COUT; p < 128; p += PARTS) bsum += __bfloat162float(s_d[p * WT::DS + tid % COUT]);
 #pragma unroll
@@ -351,10 +349,9 @@ __global__ void __launch_bounds__(256, COUT == 128 ? 1 : 2)
                 for (int j = 0; j < NTW; j += 2) {
                     // B (k = pixel, n = ci): stored [pixel][ci] -> ldmatrix.trans; two n-tiles
                     const int nt = ng * NTW + j + (lane >> 4);
-                    const int p = row * 18 + kw + ((lane >> 3) & 1) * 8 + (lane & 7);
+                    const int p = row * 18 + (kw ? kw + px : px0);
                     uint32_t b0, b1, b2, b3;
                     ldsm_x4_t(smem_u32(s_i + p * WT::IS + nt * 8), b0, b1, b2, b3);
-                    if (kw == 0) b0 &= keep0, b1 &= keep8, b2 &= keep0, b3 &= keep8;
                     mma_bf16(acc[kw][j], a0, a1, a2, a3, b0, b1);
                     if (j + 1 < NTW) mma_bf16(acc[kw][j + 1], a0, a1, a2, a3, b2, b3);
                 }
