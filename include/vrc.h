@@ -354,9 +354,11 @@ void vrc_render_params_default(vrc_render_params* p, int width, int height);
 
 typedef struct {
     double samples;          /* loop iterations of all rays (the reference's sample count) */
-    double samples_fetched;  /* samples whose voxels were read (not skipped) */
+    double samples_fetched;  /* samples whose voxels were read (not skipped); may count a few twice, see skip_runs */
     double samples_shaded;   /* samples with TF alpha > 0 under shading */
-    double skip_runs;        /* runs of samples skipped through empty cells */
+    double skip_runs;        /* runs of samples skipped through empty cells: the work of this frame, which depends on
+                                how its rays were spread over lanes, and where a ray's rest was handed on from one
+                                kernel to the next differs a little from run to run, as pre-integration's reads do */
     float kernel_ms;         /* device time of the march kernel on the context stream */
     float total_ms;          /* device time from first copy-in to last copy-out */
     int device_status;       /* 0, or an internal error code from the kernel */
