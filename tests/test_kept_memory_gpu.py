@@ -141,6 +141,44 @@ def test_failing_allocations_give_the_memory_back(vrc_lib, tmp_path):
     ctx.close()
 
 
+def test_captured_frames_keep_what_they_read(vrc_lib):
+    """A graph of a frame whose maps it builds, replayed on another stream, behind
+    other work: memory given back, and the volume destroyed and the next one
+    uploaded meanwhile, do not reach it."""
+    import torch
+    ctx = v.Context(0)
+    first, second = _voxels(256, 1), _voxels(256, 3)
+    rgba = v.TransferFunction.bake([(0.0, (0, 0, 0, 0)), (0.5, (0, 0, 0, 0)), (1.0, (255, 200, 100, 60))], 256)
+    vol = v.Volume(ctx, first)
+    p = v.default_params(128, 96)
+    pos, focus, near, far = synth.orbit_camera(vol.dims, (1.0, 1.0, 1.0), 30.0, 20.0, 1.1)
+    p.camera, p.entry_exit_mode = v.make_camera(pos, focus, near=near, far=far), v.EE_ANALYTIC
+    tfs = [v.TransferFunction(ctx, rgba, (0.0, 1.0)) for _ in range(2)]
+    want = np.array(v.render(ctx, vol, tfs[0], p, out_format=v.OUT_RGBA32F)[0])
+    v.render(ctx, vol, tfs[1], p, out_format=v.OUT_RGBA32F)  # its alpha table
+    v.render(ctx, vol, tfs[0], p, out_format=v.OUT_RGBA32F)  # the maps are of the other one again
+    out, busy = torch.zeros((96, 128, 4), device="cuda"), torch.ones(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(ctx.stream)):
+        v.render_async(ctx, vol, tfs[1], p, None, None, out)
+    ctx.trim()
+    spoil = torch.full((64 << 20,), 255, dtype=torch.uint8, device="cuda")  # where the scratch would have been
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        for _ in range(60):  # some 20 ms
+            busy.mul_(1.0)
+        graph.replay()
+    vol.close()
+    other = v.Volume(ctx, second)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), want)
+    assert want.any() and bool((spoil == 255).all())
+    del graph
+    for x in (other, *tfs, ctx):
+        x.close()
+
+
 def test_a_refused_frame_does_not_count_as_one_on_another_stream(vrc_lib):
     """Volumes too large for vrc_render_noalloc's scratch (the learned form's
     probe asks first) leave their memory to the next volume, like others."""

@@ -245,6 +245,7 @@ vrc_status vrc_context_destroy(vrc_context* c) {
     cudaFree(c->d_occ_coarse);
     cudaFree(c->d_dist);
     c->kept->give_back(true);
+    for (void* p : c->captured) cudaFree(p);
     for (cudaEvent_t ev : {c->copied[0], c->copied[1], c->consumed[0], c->consumed[1], c->queued})
         if (ev) cudaEventDestroy(ev);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
@@ -471,8 +472,8 @@ vrc_status vrc_volume_destroy(vrc_volume* v) {
     if (!v) return VRC_ERR_INVALID_ARG;
     if (v->kept) cudaSetDevice(v->kept->device);
     // What read the block did so on the context's stream, where alone the next
-    // volume writes it. Frames on streams of the caller's (vrc_render_noalloc)
-    // are what cudaFree waits for. (Not a wait for the device here: it would
+    // volume writes it. Frames on streams of the caller's (vrc_render_noalloc,
+    // captured frames) are what cudaFree waits for. (Not a wait for the device here: it would
     // end any capture that another thread has under way.)
     if (v->d_block && v->kept && !v->off_stream.load())
         v->kept->put(vrc::KeptMemory::VOLUME, v->d_block, v->block_bytes, VRC_VOLUME_KEEP);
@@ -1221,6 +1222,10 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
     P.tf_wm1 = float(P.tf_width - 1);
     const size_t npix = (size_t)p->width * p->height;
     cudaStream_t s = ctx->stream;
+    // a captured frame may be replayed on any stream, as long as the caller keeps it
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    const bool captured = cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+    if (captured) vol->off_stream.store(true);
     VRC_CUDA(ctx, cudaEventRecord(ctx->ev[0], s));
     // Pinned host buffers (cudaHostAlloc / cudaHostRegister) are read and
     // written by the kernel in place through their mapped addresses (over
@@ -1342,7 +1347,8 @@ vrc_status render_impl(vrc_context* ctx, const vrc_volume* vol, const vrc_tf* tf
                 size_t bytes = 0;
                 VRC_CUDA(ctx, ctx->kept->scratch(std::max((size_t)n, vrc::occ_distance_scratch(nc)), (size_t)n, &tmp, &bytes));
                 const cudaError_t e = vrc::launch_occ_distance(ctx->d_occ, nc, ctx->d_dist, (uint8_t*)tmp, bytes, s);
-                ctx->kept->put(vrc::KeptMemory::SCRATCH, tmp, bytes, SIZE_MAX);
+                if (captured) ctx->captured.push_back(tmp);
+                else ctx->kept->put(vrc::KeptMemory::SCRATCH, tmp, bytes, SIZE_MAX);
                 VRC_CUDA(ctx, e);
                 occ_launches += vrc::occ_distance_launches(nc, bytes);
             }

@@ -292,6 +292,7 @@ struct vrc_context {
     uint8_t* d_dist = nullptr;       // occ_dist of the skip cells
     size_t dist_bytes = 0;
     std::shared_ptr<vrc::KeptMemory> kept;
+    std::vector<void*> captured;     // distance scratch of frames that a graph may replay
     std::mutex stage_lock;           // the upload that has the kept slices, the copy stream and its events
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t copied[2] = {nullptr, nullptr}, consumed[2] = {nullptr, nullptr}, queued = nullptr;
@@ -357,7 +358,7 @@ struct vrc_volume {
     std::shared_ptr<vrc::KeptMemory> kept;  // the context's
     void* d_block = nullptr;  // the allocation of the brick pool (device placement) and all min/max tables
     size_t block_bytes = 0;
-    mutable std::atomic<bool> off_stream{false};  // a frame went to a stream of the caller's
+    mutable std::atomic<bool> off_stream{false};  // a frame went, or a graph may take it, to a stream of the caller's
     float* d_bmin = nullptr;
     float* d_bmax = nullptr;
     vrc_cell_level levels[4];  // skip cells of edge 2, 4, 8 and 16 (when smaller than the brick; 2 up to 2^30 cells)
